@@ -58,6 +58,7 @@ SIGNATURES = {
     "lbgb_step_fused_rows": (_I, [_P, _P, _I, _I, _I, _I, _I, ctypes.c_double, ctypes.c_double, _I, _P]),
     "lbgb_run_fused": (_I, [_P, _P, _I, _I, _I, _D, _D, _I, _I, ctypes.POINTER(_I), _P]),
     "lbgb_steps_per_launch": (_I, [_I, _I, _I, _I]),
+    "lbgb_max_steps_per_launch": (_I, [_I, _I, _I, _I]),
     "lbgb_run_fused_sr": (_I, [_P, _P, _I, _I, _I, _D, _D, _I, _I, ctypes.c_uint, _P, ctypes.POINTER(_I), _P]),
     "lbgb_macroscopic": (_I, [_P, _P, _P, _P, _I64, _I64, _I, _P]),
     "lbgb_mass_momentum_workspace_bytes": (_SZ, []),

@@ -81,9 +81,8 @@ __device__ __forceinline__ void pull_cell(const typename C::raw *__restrict__ sr
         }
     }
     if (BC == LBGB_CAVITY_LADD && l == ny - 1) {
-        const real lid = real(6) * real(1.0 / 36.0) * u0;
-        v[CSE] += lid;  // bounce-back of NW (set above) plus the wall term, every lid node
-        v[CSW] -= lid;
+        v[CSE] = ladd_lid<1>(v[CSE], u0);  // bounce-back of NW (set above) plus the wall term, every lid node
+        v[CSW] = ladd_lid<-1>(v[CSW], u0);
     }
     if (BC == LBGB_CAVITY && l == ny - 1) {
         const int T = ny - 1;

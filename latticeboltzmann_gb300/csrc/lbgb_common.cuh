@@ -636,6 +636,14 @@ __device__ __forceinline__ float lid_term_dev(float s, float u0) {
     return fmaf(c, s, c * (float)(1u << LOG2K));
 }
 
+// The wall-density-1 lid, g +/- 6 w u0, rounded once (SIGN +1 or -1).  Left to
+// the compiler, some kernels fused the product into the addition and some did
+// not, and their results differed in the last place.
+template <int SIGN, class R>
+__device__ __forceinline__ R ladd_lid(R g, R u0) {
+    return Ieee<R>::fma(R(SIGN) * (R(6) * R(1.0 / 36.0)), u0, g);
+}
+
 // Equilibrium of one node (same formulation as above).
 template <class R>
 __device__ __forceinline__ void equilibrium1(R rho, R ux, R uy, R (&feq)[9]) {

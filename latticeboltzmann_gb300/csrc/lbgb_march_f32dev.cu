@@ -1,0 +1,5 @@
+#include "lbgb_march.cuh"
+
+namespace lbgb {
+template int launch_march<LBGB_F32DEV>(const MarchCall &c, cudaStream_t s);
+}

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__((NCW_ + 1) * 32, PipeShape<DT>::CTAS)
 k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>::raw *__restrict__ dst, int nx,
             int ny, int tiles_per_row, int total_tiles, int stages, typename Codec<DT>::real omega,
             typename Codec<DT>::real u0, long long wait_limit, int stall_producer,
-            const unsigned long long *__restrict__ sr_step, uint32_t sr_seed, int k_first) {
+            const unsigned long long *__restrict__ sr_step, uint32_t sr_seed, uint32_t sr_offset, int k_first) {
     using C = Codec<DT>;
     using raw = typename C::raw;
     using real = typename C::real;
@@ -309,10 +309,10 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
             if (c + NC == ny) {
                 const int T = ny - 1;
                 if (BC == LBGB_CAVITY_LADD) {
-                    const real lid = real(6) * real(1.0 / 36.0) * u0 * real(1u << LOG2K);
+                    const real us = u0 * real(1u << LOG2K);
                     v[CS][NC - 1] = g(CN, k, T);
-                    v[CSE][NC - 1] = g(CNW, k, T) + lid;
-                    v[CSW][NC - 1] = g(CNE, k, T) - lid;
+                    v[CSE][NC - 1] = ladd_lid<1>(g(CNW, k, T), us);
+                    v[CSW][NC - 1] = ladd_lid<-1>(g(CNE, k, T), us);
                 } else {
                     const int kw = (k == 0) ? nx - 1 : k - 1;
                     const int ke = (k == nx - 1) ? 0 : k + 1;
@@ -386,7 +386,7 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
             }
             uint32_t base[NC / 2];
             if constexpr (sr) {
-                const uint32_t key = sr_step_key(sr_seed, *sr_step);
+                const uint32_t key = sr_step_key(sr_seed, *sr_step + sr_offset);
                 const uint32_t cell0 = (uint32_t)((size_t)k * ny + c);
 #pragma unroll
                 for (int q = 0; q < NC / 2; ++q) base[q] = sr_pair_base(key, cell0 + 2 * q);

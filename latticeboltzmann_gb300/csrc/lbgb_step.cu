@@ -23,6 +23,7 @@
 #include <stdio.h>
 
 #include "lbgb_common.cuh"
+#include "lbgb_march.h"
 #include "lbgb_pipe.cuh"
 
 namespace lbgb {
@@ -115,7 +116,7 @@ __device__ __forceinline__ void step_segment(const typename Codec<DT>::raw *__re
                                              int l0, int lane, typename Codec<DT>::real omega,
                                              typename Codec<DT>::real u0,
                                              const unsigned long long *__restrict__ sr_step, uint32_t sr_seed,
-                                             uint32_t cell_base) {
+                                             uint32_t cell_base, uint32_t sr_offset = 0) {
     using C = Codec<DT>;
     using real = typename C::real;
     using raw = typename C::raw;
@@ -151,10 +152,9 @@ __device__ __forceinline__ void step_segment(const typename Codec<DT>::raw *__re
         if (l0 + V == ny) {
             if (BC == LBGB_CAVITY_LADD) {
                 // standard Ladd wall, density 1: -/+ 6 w u0 at every lid node
-                const real lid = real(6) * real(1.0 / 36.0) * u0;
                 v[CS][V - 1] = load_one<C>(src, cs, ny, CN, k, ny - 1);
-                v[CSE][V - 1] = load_one<C>(src, cs, ny, CNW, k, ny - 1) + lid;
-                v[CSW][V - 1] = load_one<C>(src, cs, ny, CNE, k, ny - 1) - lid;
+                v[CSE][V - 1] = ladd_lid<1>(load_one<C>(src, cs, ny, CNW, k, ny - 1), u0);
+                v[CSW][V - 1] = ladd_lid<-1>(load_one<C>(src, cs, ny, CNE, k, ny - 1), u0);
             } else {
                 // lid: S bounces back; SE/SW get the Ladd term 6 w rho_lid u0,
                 // except at the corner where the side wall wins (plain bounce-back)
@@ -181,7 +181,7 @@ __device__ __forceinline__ void step_segment(const typename Codec<DT>::raw *__re
     if (COLLIDE) {
         uint32_t key = 0;
         if constexpr (sizeof(raw) == 2) {
-            if (sr_step) key = sr_step_key(sr_seed, *sr_step);
+            if (sr_step) key = sr_step_key(sr_seed, *sr_step + sr_offset);
         }
 #pragma unroll
         for (int j = 0; j < V; ++j) {
@@ -216,14 +216,14 @@ template <int DT, int BC, bool COLLIDE, int V>
 __global__ void __launch_bounds__(256, min_blocks<DT, V>())
 k_step(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>::raw *__restrict__ dst, int nx,
        int ny, int segs, long long tasks, typename Codec<DT>::real omega, typename Codec<DT>::real u0,
-       const unsigned long long *__restrict__ sr_step, uint32_t sr_seed, int k_first) {
+       const unsigned long long *__restrict__ sr_step, uint32_t sr_seed, uint32_t sr_offset, int k_first) {
     const int lane = threadIdx.x & 31;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tasks; t += nwarps) {
         const int kr = (int)(t / segs);
         const int k = k_first + kr;
         const int l0 = (int)(t - (long long)kr * segs) * (32 * V) + lane * V;
-        step_segment<DT, BC, COLLIDE, V>(src, dst, nx, ny, k, l0, lane, omega, u0, sr_step, sr_seed, 0u);
+        step_segment<DT, BC, COLLIDE, V>(src, dst, nx, ny, k, l0, lane, omega, u0, sr_step, sr_seed, 0u, sr_offset);
     }
 }
 
@@ -244,6 +244,7 @@ static int sm_count() {
 struct SR {
     const unsigned long long *step = nullptr;  // device step counter; null: round to nearest
     uint32_t seed = 0;
+    uint32_t offset = 0;  // steps taken since the counter was last advanced
 };
 
 // Rows [first, first + count) of the lattice to update (count < 0: all).
@@ -267,7 +268,7 @@ static int launch_v(const void *src, void *dst, int nx, int ny, double omega, do
     if (blocks > cap) blocks = cap;
     k_step<DT, BC, COLLIDE, V><<<(unsigned)blocks, threads, 0, s>>>(
         static_cast<const typename C::raw *>(src), static_cast<typename C::raw *>(dst), nx, ny, segs, tasks,
-        (typename C::real)omega, (typename C::real)u0, sr.step, sr.seed, rows.first);
+        (typename C::real)omega, (typename C::real)u0, sr.step, sr.seed, sr.offset, rows.first);
     return check_launch("k_step");
 }
 
@@ -278,7 +279,7 @@ struct Tuning {
     long long wait_limit = 1ll << 22;    // tries per bounded mbarrier wait
     long long pipe_min_cells = 1 << 16;  // auto: smaller lattices use the register kernel
     long long stall_producer = 0;        // test hook: the producer delivers nothing
-    long long two_step = 1;              // auto kernel: two time steps per launch where k_step2 applies
+    long long two_step = 1;              // auto kernel: several time steps per launch where k_march applies
 };
 static Tuning g_tune;
 
@@ -295,63 +296,48 @@ static int max_dyn_smem() {
     return v;
 }
 
-}  // namespace lbgb
-#include "lbgb_step2.cuh"
-namespace lbgb {
-
-// Rows per block of the two-step kernel: the largest of 128, 64, 32, 16 that
-// divides nx (0: none does).
-static int step2_rows(int nx) {
-    for (int r = 128; r >= 16; r /= 2)
-        if (nx % r == 0) return r;
-    return 0;
+// Lattices that the multi-step march takes: every storage but FP64 (whose
+// collision the FP64 units bound, not memory).  Rows without whole 16-byte
+// vectors go element by element, for 4-byte codes only.  Below 2048 cells one
+// launch per step is as fast.
+static bool march_applies(const void *src, const void *dst, int nx, int ny, int dtype, bool &ragged) {
+    if (!g_tune.two_step || g_tune.kernel != 0 || dtype == LBGB_F64) return false;
+    if (nx < 8 || ny < 16 || (long long)nx * ny < (1 << 11)) return false;
+    const int es = (int)raw_size(dtype);
+    ragged = ny % (16 / es) != 0 || (src && !aligned(src, 16)) || (dst && !aligned(dst, 16));
+    return !ragged || es == 4;
 }
 
-static bool step2_applies(const void *src, const void *dst, int nx, int ny, int boundary, int dtype) {
-    // 16-bit codes stay on the single-step kernel: issue-bound already, they
-    // measured slower with two steps per launch (8192^2 cavity: 148k against
-    // 169k MLUPS FP16, 149k against 171k BF16)
-    return g_tune.two_step && g_tune.kernel == 0 && (dtype == LBGB_F32 || dtype == LBGB_F32DEV) &&
-           (boundary == LBGB_PERIODIC || boundary == LBGB_CAVITY) && step2_rows(nx) && ny % S2_W == 0 &&
-           ny / S2_W <= 65535 && (!src || aligned(src, 16)) && (!dst || aligned(dst, 16));
+// Steps of one launch, of `left` still to do: four per pass from 1.5 M cells
+// on (8192^2 FP32 cavity: 252k MLUPS against 155k with two, 2048^2 160k against
+// 125k); below that the two extra rows a side of every chunk cost more than
+// the pass saves (1024^2 99k against 110k).
+static int march_steps(int nx, int ny, int left) {
+    return left >= 4 && (long long)nx * ny >= 1500000 ? 4 : (left >= 2 ? 2 : 1);
 }
 
-template <int DT, int BC>
-static int launch_step2(const void *src, void *dst, int nx, int ny, double omega, double u0, cudaStream_t s) {
-    using raw = typename Codec<DT>::raw;
-    static std::atomic<bool> attr_set[MAX_DEVICES];
-    const int dev = current_device();
-    if (!attr_set[dev].load(std::memory_order_acquire)) {
-        std::lock_guard<std::mutex> lock(setup_mutex());
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_step2<DT, BC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S2Geom<raw>::SMEM);
-        if (e != cudaSuccess) {
-            set_error("k_step2: cannot reserve %zu bytes of shared memory: %s", S2Geom<raw>::SMEM,
-                      cudaGetErrorString(e));
-            return LBGB_ECUDA;
-        }
-        attr_set[dev].store(true, std::memory_order_release);
-    }
-    const int rows = step2_rows(nx);
-    k_step2<DT, BC><<<dim3(nx / rows, ny / S2_W), S2_THREADS, S2Geom<raw>::SMEM, s>>>(
-        static_cast<const raw *>(src), static_cast<raw *>(dst), nx, ny, rows, (typename Codec<DT>::real)omega,
-        (typename Codec<DT>::real)u0);
-    return check_launch("k_step2");
-}
-
-// Two fused steps src -> dst in one launch; 1 (nothing launched) where the
-// two-step kernel does not apply.
-static int step2(const void *src, void *dst, int nx, int ny, int boundary, double omega, double u0, int dtype,
-                 cudaStream_t s) {
-    if (!step2_applies(src, dst, nx, ny, boundary, dtype)) return 1;
-    const bool cav = boundary == LBGB_CAVITY;
+// 2 or 4 fused steps src -> dst in one launch.
+static int march(const void *src, void *dst, int nx, int ny, int boundary, double omega, double u0, int dtype,
+                 int steps, bool ragged, SR sr, cudaStream_t s) {
+    MarchCall c;
+    c.src = src;
+    c.dst = dst;
+    c.nx = nx;
+    c.ny = ny;
+    c.boundary = boundary;
+    c.steps = steps;
+    c.ragged = ragged;
+    c.omega = omega;
+    c.u0 = boundary == LBGB_PERIODIC ? 0.0 : u0;
+    c.sr_step = sr.step;
+    c.sr_seed = sr.seed;
+    c.sr_offset = sr.offset;
+    c.sms = sm_count();
     switch (dtype) {
-    case LBGB_F32:
-        return cav ? launch_step2<LBGB_F32, LBGB_CAVITY>(src, dst, nx, ny, omega, u0, s)
-                   : launch_step2<LBGB_F32, LBGB_PERIODIC>(src, dst, nx, ny, omega, 0.0, s);
-    default:
-        return cav ? launch_step2<LBGB_F32DEV, LBGB_CAVITY>(src, dst, nx, ny, omega, u0, s)
-                   : launch_step2<LBGB_F32DEV, LBGB_PERIODIC>(src, dst, nx, ny, omega, 0.0, s);
+    case LBGB_F32: return launch_march<LBGB_F32>(c, s);
+    case LBGB_F32DEV: return launch_march<LBGB_F32DEV>(c, s);
+    case LBGB_F16DEV: return launch_march<LBGB_F16DEV>(c, s);
+    default: return launch_march<LBGB_BF16DEV>(c, s);
     }
 }
 
@@ -388,7 +374,7 @@ static int launch_pipe(const void *src, void *dst, int nx, int ny, double omega,
         kernel<<<grid, (SH::NCW + 1) * 32, smem, s>>>(
             static_cast<const raw *>(src), static_cast<raw *>(dst), nx, ny, (int)tpr, (int)total, stages,
             (typename Codec<DT>::real)omega, (typename Codec<DT>::real)u0, g_tune.wait_limit,
-            (int)g_tune.stall_producer, sr.step, sr.seed, rows.first);
+            (int)g_tune.stall_producer, sr.step, sr.seed, sr.offset, rows.first);
         return LBGB_OK;
     };
     const int rc = srnd ? go(k_step_pipe<DT, BC, COLLIDE, SH::NCW, SH::NC, sizeof(raw) == 2 && COLLIDE>, 1)
@@ -518,19 +504,14 @@ extern "C" int lbgb_run_fused(void *a, void *b, int nx, int ny, int boundary, do
     int rc = check_grid(a, b, nx, ny, dtype, boundary, "lbgb_run_fused");
     if (rc) return rc;
     void *src = a, *dst = b;
-    int s = 0;
-    // pairs of steps in one launch each where the two-step kernel applies
-    for (; s + 1 < nsteps; s += 2) {
-        rc = step2(src, dst, nx, ny, boundary, omega, u0, dtype, (cudaStream_t)stream);
-        if (rc > 0) break;
-        if (rc < 0) return rc;
-        void *t = src;
-        src = dst;
-        dst = t;
-    }
-    for (; s < nsteps; ++s) {
-        rc = lbgb_step_fused(src, dst, nx, ny, boundary, omega, u0, dtype, stream);
+    bool ragged = false;
+    const bool several = march_applies(a, b, nx, ny, dtype, ragged);
+    for (int left = nsteps; left > 0;) {
+        const int n = several ? march_steps(nx, ny, left) : 1;
+        rc = n > 1 ? march(src, dst, nx, ny, boundary, omega, u0, dtype, n, ragged, SR(), (cudaStream_t)stream)
+                   : lbgb_step_fused(src, dst, nx, ny, boundary, omega, u0, dtype, stream);
         if (rc) return rc;
+        left -= n;
         void *t = src;
         src = dst;
         dst = t;
@@ -540,11 +521,20 @@ extern "C" int lbgb_run_fused(void *a, void *b, int nx, int ny, int boundary, do
 }
 
 extern "C" int lbgb_steps_per_launch(int nx, int ny, int boundary, int dtype) {
-    return step2_applies(nullptr, nullptr, nx, ny, boundary, dtype) ? 2 : 1;
+    return g_tune.two_step && g_tune.kernel == 0 && (dtype == LBGB_F32 || dtype == LBGB_F32DEV) &&
+                   (boundary == LBGB_PERIODIC || boundary == LBGB_CAVITY) && nx % 16 == 0 && ny % 128 == 0
+               ? 2
+               : 1;
+}
+
+extern "C" int lbgb_max_steps_per_launch(int nx, int ny, int boundary, int dtype) {
+    bool ragged = false;
+    if (raw_size(dtype) == 0 || boundary < LBGB_PERIODIC || boundary > LBGB_CAVITY_LADD) return 1;
+    return march_applies(nullptr, nullptr, nx, ny, dtype, ragged) ? march_steps(nx, ny, 4) : 1;
 }
 
 namespace lbgb {
-__global__ void k_bump_step(unsigned long long *ctr) { *ctr += 1; }
+__global__ void k_bump_step(unsigned long long *ctr, unsigned long long n) { *ctr += n; }
 }  // namespace lbgb
 
 #include "lbgb_batch.cuh"
@@ -569,17 +559,27 @@ extern "C" int lbgb_run_fused_sr(void *a, void *b, int nx, int ny, int boundary,
     sr.step = step_counter;
     sr.seed = seed;
     void *src = a, *dst = b;
-    for (int i = 0; i < nsteps; ++i) {
-        rc = boundary == LBGB_CAVITY        ? dispatch<LBGB_CAVITY, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
-             : boundary == LBGB_CAVITY_LADD ? dispatch<LBGB_CAVITY_LADD, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
-                                            : dispatch<LBGB_PERIODIC, true>(src, dst, nx, ny, dtype, omega, 0.0, s, sr);
+    bool ragged = false;
+    const bool several = march_applies(a, b, nx, ny, dtype, ragged);
+    for (int left = nsteps; left > 0;) {
+        const int n = several ? march_steps(nx, ny, left) : 1;
+        sr.offset = (uint32_t)(nsteps - left);
+        rc = n > 1 ? march(src, dst, nx, ny, boundary, omega, u0, dtype, n, ragged, sr, s)
+             : boundary == LBGB_CAVITY
+                 ? dispatch<LBGB_CAVITY, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
+             : boundary == LBGB_CAVITY_LADD
+                 ? dispatch<LBGB_CAVITY_LADD, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
+                 : dispatch<LBGB_PERIODIC, true>(src, dst, nx, ny, dtype, omega, 0.0, s, sr);
         if (rc) return rc;
-        k_bump_step<<<1, 1, 0, s>>>(step_counter);
-        rc = check_launch("k_bump_step");
-        if (rc) return rc;
+        left -= n;
         void *t = src;
         src = dst;
         dst = t;
+    }
+    if (nsteps > 0) {
+        k_bump_step<<<1, 1, 0, s>>>(step_counter, (unsigned long long)nsteps);
+        rc = check_launch("k_bump_step");
+        if (rc) return rc;
     }
     if (which) *which = (src == a) ? 0 : 1;
     return LBGB_OK;

@@ -106,18 +106,22 @@ class Lattice:
 
     @property
     def bytes_per_cell_update(self):
-        """Algorithmic HBM bytes per cell and launch: 9 loads + 9 stores (one
-        step per launch; two where ``steps_per_launch`` is 2)."""
+        """Algorithmic HBM bytes per cell and launch: 9 loads + 9 stores (of
+        one step or of several, see ``step``)."""
         return 18 * self._buf[0].element_size()
 
     @property
     def steps_per_launch(self):
-        """Steps that ``step(n)`` advances per launch for n >= 2: 2 where the
-        two-step kernel applies to this lattice (FP32 or f32dev storage,
-        periodic or cavity walls, nx a multiple of 16, ny of 128), else 1."""
+        """2 for lattices whose steps ``step(n)`` is sure to pair whatever their
+        size (FP32 or f32dev storage, periodic or cavity walls, nx a multiple of
+        16, ny of 128), else 1; larger lattices advance up to four steps per
+        launch (``lbgb_max_steps_per_launch``)."""
         if self.rounding == "stochastic" and self.storage in ("f16dev", "bf16dev"):
             return 1
         return int(_lib.load().lbgb_steps_per_launch(self.nx, self.ny, self.bcode, self.code))
+
+    def _max_steps_per_launch(self):
+        return int(_lib.load().lbgb_max_steps_per_launch(self.nx, self.ny, self.bcode, self.code))
 
     @property
     def state(self):
@@ -314,7 +318,8 @@ class Lattice:
 
     # ------------------------------------------------------------------ stepping
     def step(self, n=1):
-        """Advance ``n`` time steps (one fused launch each)."""
+        """Advance ``n`` time steps: fused launches of one, two or four steps
+        each (one read and one write of the lattice per launch)."""
         if n <= 0:
             return self
         which = ctypes.c_int(0)
@@ -350,16 +355,22 @@ class Lattice:
                       self.omega, self.u0, self.code, 1, self.seed, ctr.data_ptr(), ctypes.byref(ctypes.c_int(0)),
                       self._stream())
         torch.cuda.current_stream(self.device).synchronize()
-        s = torch.cuda.Stream(device=self.device)
-        s.wait_stream(torch.cuda.current_stream(self.device))
-        g = torch.cuda.CUDAGraph()
         cur = self._cur
-        with torch.cuda.stream(s):
-            with torch.cuda.graph(g, stream=s):
-                self.step(n)
-        # capture recorded launches only; restore the bookkeeping
-        self._cur = cur
-        self.steps_taken -= n
+        # an odd number of launches of several steps each would leave the
+        # state in the other buffer: the last one is then split in two
+        last = 4 if n % 4 == 0 and self._max_steps_per_launch() == 4 else 2
+        for parts in ((n,), (n - last, last // 2, last // 2)):
+            s = torch.cuda.Stream(device=self.device)
+            s.wait_stream(torch.cuda.current_stream(self.device))
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.stream(s):
+                with torch.cuda.graph(g, stream=s):
+                    for p in parts:
+                        self.step(p)
+            self.steps_taken -= n
+            if self._cur == cur:
+                break
+            self._cur = cur
         torch.cuda.current_stream(self.device).wait_stream(s)
         lattice = self
 
