@@ -12,6 +12,7 @@
 #include <mutex>
 
 #include "lbgb.h"
+#include "lbgb_fix64.cuh"
 
 namespace lbgb {
 
@@ -741,9 +742,12 @@ __device__ __forceinline__ void collide_encode(typename Codec<DT>::real (&f)[9],
         }
         out[0] = C::enc_h(dm);
     } else {
-        bgk_collide(f, omega);
+        fix64::Factor k;
+        if (!fix64::omega_factor(omega, k) || !fix64::collide(f, k, out)) {
+            bgk_collide(f, omega);
 #pragma unroll
-        for (int i = 0; i < 9; ++i) out[i] = C::enc(f[i], i);
+            for (int i = 0; i < 9; ++i) out[i] = f[i];
+        }
     }
 }
 

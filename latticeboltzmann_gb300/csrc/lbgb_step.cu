@@ -258,9 +258,10 @@ template <int DT, int BC, bool COLLIDE, int V>
 static int launch_v(const void *src, void *dst, int nx, int ny, double omega, double u0, cudaStream_t s,
                     SR sr = SR(), Rows rows = Rows()) {
     using C = Codec<DT>;
-    const int threads = 256;
     const int segs = (ny + 32 * V - 1) / (32 * V);
     const long long tasks = (long long)rows.n(nx) * segs;
+    // small lattices in blocks of two warps, which reach every SM
+    const int threads = tasks < 16ll * sm_count() ? 64 : 256;
     const long long warps_per_block = threads / 32;
     long long blocks = (tasks + warps_per_block - 1) / warps_per_block;
     // at most 16 resident-size waves of blocks; the rest is grid-stride
@@ -397,6 +398,9 @@ static int launch(const void *src, void *dst, int nx, int ny, double omega, doub
         const int rc = launch_pipe<DT, BC, COLLIDE>(src, dst, nx, ny, omega, u0, s, sr, rows);
         if (rc <= 0) return rc;
     }
+    // FP64 lattices that leave SMs idle with two cells per lane: one per lane
+    if (DT == LBGB_F64 && (long long)rows.n(nx) * ny < 1024ll * sm_count())
+        return launch_v<DT, BC, COLLIDE, 1>(src, dst, nx, ny, omega, u0, s, sr, rows);
     if (vec_ok) return launch_v<DT, BC, COLLIDE, VW>(src, dst, nx, ny, omega, u0, s, sr, rows);
     return launch_v<DT, BC, COLLIDE, 1>(src, dst, nx, ny, omega, u0, s, sr, rows);
 }
