@@ -3,8 +3,8 @@
 
 Workload (default): lid-driven cavity, 8192 x 8192 cells, FP32 populations,
 omega = 1.7, lid velocity 0.1, from rest at equilibrium.  One step = one
-fused pull-stream + collide update of the whole lattice; the solver runs up
-to four steps per kernel launch (every storage but FP64: one read and one
+fused pull-stream + collide update of the whole lattice; the solver runs
+several steps per kernel launch (four at the default size: one read and one
 write of the lattice per launch).
 Metric: MLUPS (million lattice-cell updates per second, physical cells only).
 
@@ -210,7 +210,7 @@ def steps_per_event(lat, steps):
     """The most steps that one launch advances, of those that divide ``steps``."""
     from latticeboltzmann_gb300 import _lib
     most = int(_lib.load().lbgb_max_steps_per_launch(lat.nx, lat.ny, lat.bcode, lat.code))
-    return next(c for c in (4, 2, 1) if c <= most and steps % c == 0)
+    return next(c for c in range(most, 0, -1) if steps % c == 0)
 
 
 def profiled_traffic(storage, boundary, cells, kernel="k_step_pipe"):
@@ -480,7 +480,7 @@ def run_ours(args):
                 "frac": round(achieved / peak, 4), "traffic": None if traffic is None else round(traffic),
                 "algorithmic_bytes": bpc * lat.cells, "steps_per_launch": chunk,
                 "bytes_per_cell_update": bpc / chunk,
-                "kernel": ("k_march (%d fused steps per launch: pull stream + bounce-back/lid + BGK, the "
+                "kernel": ("k_march / k_tile (%d fused steps per launch: pull stream + bounce-back/lid + BGK, the "
                            "intermediate steps on chip)" % chunk if chunk > 1 else
                            "k_step (fused pull stream + bounce-back/lid + BGK)"),
                 "peak_source": peak_src,

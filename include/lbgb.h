@@ -165,11 +165,11 @@ LBGB_API int lbgb_step_fused_rows(const void *src, void *dst, int nx, int ny, in
 /* nsteps fused steps ping-ponging between a and b (a holds the initial
  * state); *which receives 0 if the result is in a, 1 if in b.  Launch-only:
  * suitable for CUDA-graph capture.  With the auto kernel and
- * LBGB_TUNE_TWO_STEP on, lattices of 2048 cells and more (nx >= 8, ny >= 16,
- * every storage but LBGB_F64; 16-bit codes need ny a multiple of 8 and 16-byte
- * aligned buffers) advance two or four steps per launch, the intermediate
- * steps kept on chip (k_march: one read and one write of the lattice per
- * launch); the results equal single steps bit for bit. */
+ * LBGB_TUNE_TWO_STEP on, most lattices advance several steps per launch, the
+ * intermediate steps kept on chip: up to eight for small ones (k_tile), two or
+ * four for large ones of every storage but LBGB_F64 (k_march; 16-bit codes need
+ * ny a multiple of 8 and 16-byte aligned buffers).  The results equal single
+ * steps bit for bit. */
 LBGB_API int lbgb_run_fused(void *a, void *b, int nx, int ny, int boundary,
                    double omega, double u0, int dtype, int nsteps, int *which,
                    void *stream);
@@ -180,8 +180,8 @@ LBGB_API int lbgb_run_fused(void *a, void *b, int nx, int ny, int boundary,
  * lattices take more steps (lbgb_max_steps_per_launch). */
 LBGB_API int lbgb_steps_per_launch(int nx, int ny, int boundary, int dtype);
 
-/* The most steps lbgb_run_fused advances per launch on this lattice (1, 2 or
- * 4; 16-byte aligned buffers). */
+/* The most steps lbgb_run_fused advances per launch on this lattice (1 to 8;
+ * 16-byte aligned buffers, rounding to nearest). */
 LBGB_API int lbgb_max_steps_per_launch(int nx, int ny, int boundary, int dtype);
 
 /* As lbgb_run_fused, with stochastic rounding of the 16-bit storage codes
@@ -427,8 +427,8 @@ LBGB_API int lbgb_fno_sum_splits(const float *parts, float *out, int S, long lon
  *   LBGB_TUNE_WAIT_LIMIT      tries per bounded device-side wait
  *   LBGB_TUNE_PIPE_MIN_CELLS  auto: lattices with fewer cells use the register kernel
  *   LBGB_TUNE_TWO_STEP        1 (default): with the auto kernel, lbgb_run_fused advances
- *                             two or four steps in one launch (per read and write of the
- *                             lattice) where that kernel applies; 0: one step per launch
+ *                             several steps in one launch (per read and write of the
+ *                             lattice) where those kernels apply; 0: one step per launch
  *   LBGB_TUNE_TEST_STALL_PRODUCER  test hook: the pipelined kernel's producer
  *                             delivers nothing, so its consumers' bounded
  *                             waits expire (exercises the timeout path)

@@ -644,6 +644,11 @@ template <int SIGN, class R>
 __device__ __forceinline__ R ladd_lid(R g, R u0) {
     return Ieee<R>::fma(R(SIGN) * (R(6) * R(1.0 / 36.0)), u0, g);
 }
+// The half-precision kernels that collide in stored units (the pipelined
+// kernel and those that stand in for it) round the product on its own.
+__device__ __forceinline__ float ladd_term_units(float u0) {
+    return __fmul_rn(6.f * (float)(1.0 / 36.0), u0) * F16_SCALE;
+}
 
 // Equilibrium of one node (same formulation as above).
 template <class R>

@@ -150,9 +150,9 @@ __device__ __forceinline__ Lid march_edges(uint32_t (&v)[9][4], const uint32_t (
     }
     if (top) {
         if (BC == LBGB_CAVITY_LADD) {
-            // as ladd_lid: one fused operation in march_collide
-            lid.coef = 6.f * (float)(1.0 / 36.0);
-            lid.term = u0 * (float)(1u << PC::LOG2K);
+            // as ladd_lid (one fused operation in march_collide) or, in units, ladd_term_units
+            lid.coef = PC::LOG2K ? 1.f : 6.f * (float)(1.0 / 36.0);
+            lid.term = PC::LOG2K ? ladd_term_units(u0) : u0;
             lid.se = lid.sw = true;
         } else {
             // the single-step kernel's sum order

@@ -1,5 +1,7 @@
 #include "lbgb_march.cuh"
+#include "lbgb_tile.cuh"
 
 namespace lbgb {
 template int launch_march<LBGB_BF16DEV>(const MarchCall &c, cudaStream_t s);
-}
+template int launch_tile<LBGB_BF16DEV>(const TileCall &c, cudaStream_t s);
+}  // namespace lbgb

@@ -1,0 +1,5 @@
+#include "lbgb_tile.cuh"
+
+namespace lbgb {
+template int launch_tile<LBGB_F64>(const TileCall &c, cudaStream_t s);
+}  // namespace lbgb

@@ -309,10 +309,14 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
             if (c + NC == ny) {
                 const int T = ny - 1;
                 if (BC == LBGB_CAVITY_LADD) {
-                    const real us = u0 * real(1u << LOG2K);
                     v[CS][NC - 1] = g(CN, k, T);
-                    v[CSE][NC - 1] = ladd_lid<1>(g(CNW, k, T), us);
-                    v[CSW][NC - 1] = ladd_lid<-1>(g(CNE, k, T), us);
+                    if constexpr (UNITS) {
+                        v[CSE][NC - 1] = g(CNW, k, T) + ladd_term_units(u0);
+                        v[CSW][NC - 1] = g(CNE, k, T) - ladd_term_units(u0);
+                    } else {
+                        v[CSE][NC - 1] = ladd_lid<1>(g(CNW, k, T), u0);
+                        v[CSW][NC - 1] = ladd_lid<-1>(g(CNE, k, T), u0);
+                    }
                 } else {
                     const int kw = (k == 0) ? nx - 1 : k - 1;
                     const int ke = (k == nx - 1) ? 0 : k + 1;

@@ -25,6 +25,7 @@
 #include "lbgb_common.cuh"
 #include "lbgb_march.h"
 #include "lbgb_pipe.cuh"
+#include "lbgb_tile.h"
 
 namespace lbgb {
 
@@ -297,43 +298,85 @@ static int max_dyn_smem() {
     return v;
 }
 
-// Lattices that the multi-step march takes: every storage but FP64 (whose
-// collision the FP64 units bound, not memory).  Rows without whole 16-byte
-// vectors go element by element, for 4-byte codes only.  Below 2048 cells one
-// launch per step is as fast.
-static bool march_applies(const void *src, const void *dst, int nx, int ny, int dtype, bool &ragged) {
-    if (!g_tune.two_step || g_tune.kernel != 0 || dtype == LBGB_F64) return false;
-    if (nx < 8 || ny < 16 || (long long)nx * ny < (1 << 11)) return false;
+// How lbgb_run_fused advances a lattice.
+struct Several {
+    enum { ONE, MARCH, TILE } kind = ONE;
+    int most = 1;         // steps of one launch
+    bool ragged = false;  // MARCH: rows without whole 16-byte vectors
+    const TilePlan *plan = nullptr;
+};
+
+// Tiles up to the sizes where the march (4-byte codes 0.95 M cells, 1.5 M
+// without whole vectors; 16-bit codes 1.1 M) or, for FP64, one step per launch
+// (150 k cells) is as fast; 16-bit rows without whole vectors always, as the
+// march does not take them.  The march: every storage but FP64; four steps per
+// pass from 1.5 M cells on (8192^2 FP32 cavity 252k MLUPS against 155k with
+// two, 2048^2 160k against 125k), below that two, since the two rows a side
+// that each step adds to a chunk then cost more than the pass saves (1024^2 99k
+// against 110k).
+static Several several_steps(const void *src, const void *dst, int nx, int ny, int dtype, bool sr) {
+    Several m;
     const int es = (int)raw_size(dtype);
-    ragged = ny % (16 / es) != 0 || (src && !aligned(src, 16)) || (dst && !aligned(dst, 16));
-    return !ragged || es == 4;
+    if (!g_tune.two_step || g_tune.kernel != 0 || es == 0) return m;
+    const long long cells = (long long)nx * ny;
+    m.ragged = ny % (16 / es) != 0 || (src && !aligned(src, 16)) || (dst && !aligned(dst, 16));
+    const long long tile_most = dtype == LBGB_F64 ? 150000
+                                : es == 2         ? (m.ragged ? (long long)INT_MAX : 1100000)
+                                                  : (m.ragged ? 1500000 : 950000);
+    if (nx >= 2 && ny >= 2 && cells <= tile_most) {
+        // the plans of the last few kinds of lattice of this host thread
+        thread_local TilePlan plans[8];
+        thread_local int next = 0;
+        const int kind = 2 * dtype + (sr ? 1 : 0), sms = sm_count();
+        for (const TilePlan &p : plans)
+            if (p.nx == nx && p.ny == ny && p.kind == kind && p.sms == sms) m.plan = &p;
+        if (!m.plan) {
+            TilePlan &p = plans[next];
+            next = (next + 1) % 8;
+            tile_plan(p, nx, ny, kind, es, dtype == LBGB_F64 ? 13.5 : (sr ? 4.0 : 1.45), sms);
+            m.plan = &p;
+        }
+        if (m.plan->steps > 1) {
+            m.kind = Several::TILE;
+            m.most = m.plan->steps;
+            return m;
+        }
+    }
+    if (dtype == LBGB_F64 || nx < 8 || ny < 16 || cells < 2048 || (m.ragged && es != 4)) return m;
+    m.kind = Several::MARCH;
+    m.most = cells >= 1500000 ? 4 : 2;
+    return m;
 }
 
-// Steps of one launch, of `left` still to do: four per pass from 1.5 M cells
-// on (8192^2 FP32 cavity: 252k MLUPS against 155k with two, 2048^2 160k against
-// 125k); below that the two extra rows a side of every chunk cost more than
-// the pass saves (1024^2 99k against 110k).
-static int march_steps(int nx, int ny, int left) {
-    return left >= 4 && (long long)nx * ny >= 1500000 ? 4 : (left >= 2 ? 2 : 1);
+// `left` steps to do: as many launches as it takes, of about equal length for
+// the tiles, of four and two steps (then one) for the march.
+static int next_steps(const Several &m, int left) {
+    if (m.kind == Several::TILE) {
+        const int launches = (left + m.most - 1) / m.most;
+        int n = (left + launches - 1) / launches;
+        while (n > 1 && !m.plan->shape[n].rows) --n;
+        return n;
+    }
+    if (m.kind == Several::MARCH) return m.most == 4 && left >= 4 ? 4 : (left >= 2 ? 2 : 1);
+    return 1;
 }
 
-// 2 or 4 fused steps src -> dst in one launch.
-static int march(const void *src, void *dst, int nx, int ny, int boundary, double omega, double u0, int dtype,
-                 int steps, bool ragged, SR sr, cudaStream_t s) {
-    MarchCall c;
-    c.src = src;
-    c.dst = dst;
-    c.nx = nx;
-    c.ny = ny;
-    c.boundary = boundary;
-    c.steps = steps;
-    c.ragged = ragged;
-    c.omega = omega;
-    c.u0 = boundary == LBGB_PERIODIC ? 0.0 : u0;
-    c.sr_step = sr.step;
-    c.sr_seed = sr.seed;
-    c.sr_offset = sr.offset;
-    c.sms = sm_count();
+// n > 1 fused steps src -> dst in one launch.
+static int several(const Several &m, const void *src, void *dst, int nx, int ny, int boundary, double omega, double u0,
+                   int dtype, int n, SR sr, cudaStream_t s) {
+    const double lid = boundary == LBGB_PERIODIC ? 0.0 : u0;
+    if (m.kind == Several::TILE) {
+        const TileCall c{src, dst, nx, ny, boundary, omega, lid, sr.step, sr.seed, sr.offset, m.plan->shape[n],
+                         !m.ragged && (long long)nx * ny >= g_tune.pipe_min_cells};
+        switch (dtype) {
+        case LBGB_F32: return launch_tile<LBGB_F32>(c, s);
+        case LBGB_F64: return launch_tile<LBGB_F64>(c, s);
+        case LBGB_F16DEV: return launch_tile<LBGB_F16DEV>(c, s);
+        case LBGB_BF16DEV: return launch_tile<LBGB_BF16DEV>(c, s);
+        default: return launch_tile<LBGB_F32DEV>(c, s);
+        }
+    }
+    const MarchCall c{src, dst, nx, ny, boundary, n, m.ragged, omega, lid, sr.step, sr.seed, sr.offset, sm_count()};
     switch (dtype) {
     case LBGB_F32: return launch_march<LBGB_F32>(c, s);
     case LBGB_F32DEV: return launch_march<LBGB_F32DEV>(c, s);
@@ -508,11 +551,10 @@ extern "C" int lbgb_run_fused(void *a, void *b, int nx, int ny, int boundary, do
     int rc = check_grid(a, b, nx, ny, dtype, boundary, "lbgb_run_fused");
     if (rc) return rc;
     void *src = a, *dst = b;
-    bool ragged = false;
-    const bool several = march_applies(a, b, nx, ny, dtype, ragged);
+    const Several m = several_steps(a, b, nx, ny, dtype, false);
     for (int left = nsteps; left > 0;) {
-        const int n = several ? march_steps(nx, ny, left) : 1;
-        rc = n > 1 ? march(src, dst, nx, ny, boundary, omega, u0, dtype, n, ragged, SR(), (cudaStream_t)stream)
+        const int n = next_steps(m, left);
+        rc = n > 1 ? several(m, src, dst, nx, ny, boundary, omega, u0, dtype, n, SR(), (cudaStream_t)stream)
                    : lbgb_step_fused(src, dst, nx, ny, boundary, omega, u0, dtype, stream);
         if (rc) return rc;
         left -= n;
@@ -532,9 +574,8 @@ extern "C" int lbgb_steps_per_launch(int nx, int ny, int boundary, int dtype) {
 }
 
 extern "C" int lbgb_max_steps_per_launch(int nx, int ny, int boundary, int dtype) {
-    bool ragged = false;
-    if (raw_size(dtype) == 0 || boundary < LBGB_PERIODIC || boundary > LBGB_CAVITY_LADD) return 1;
-    return march_applies(nullptr, nullptr, nx, ny, dtype, ragged) ? march_steps(nx, ny, 4) : 1;
+    if (nx <= 0 || ny <= 0 || boundary < LBGB_PERIODIC || boundary > LBGB_CAVITY_LADD) return 1;
+    return several_steps(nullptr, nullptr, nx, ny, dtype, false).most;
 }
 
 namespace lbgb {
@@ -563,12 +604,11 @@ extern "C" int lbgb_run_fused_sr(void *a, void *b, int nx, int ny, int boundary,
     sr.step = step_counter;
     sr.seed = seed;
     void *src = a, *dst = b;
-    bool ragged = false;
-    const bool several = march_applies(a, b, nx, ny, dtype, ragged);
+    const Several m = several_steps(a, b, nx, ny, dtype, true);
     for (int left = nsteps; left > 0;) {
-        const int n = several ? march_steps(nx, ny, left) : 1;
+        const int n = next_steps(m, left);
         sr.offset = (uint32_t)(nsteps - left);
-        rc = n > 1 ? march(src, dst, nx, ny, boundary, omega, u0, dtype, n, ragged, sr, s)
+        rc = n > 1 ? several(m, src, dst, nx, ny, boundary, omega, u0, dtype, n, sr, s)
              : boundary == LBGB_CAVITY
                  ? dispatch<LBGB_CAVITY, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
              : boundary == LBGB_CAVITY_LADD

@@ -114,8 +114,8 @@ class Lattice:
     def steps_per_launch(self):
         """2 for lattices whose steps ``step(n)`` is sure to pair whatever their
         size (FP32 or f32dev storage, periodic or cavity walls, nx a multiple of
-        16, ny of 128), else 1; larger lattices advance up to four steps per
-        launch (``lbgb_max_steps_per_launch``)."""
+        16, ny of 128), else 1; most lattices advance more steps per launch
+        (``lbgb_max_steps_per_launch``)."""
         if self.rounding == "stochastic" and self.storage in ("f16dev", "bf16dev"):
             return 1
         return int(_lib.load().lbgb_steps_per_launch(self.nx, self.ny, self.bcode, self.code))
@@ -318,8 +318,8 @@ class Lattice:
 
     # ------------------------------------------------------------------ stepping
     def step(self, n=1):
-        """Advance ``n`` time steps: fused launches of one, two or four steps
-        each (one read and one write of the lattice per launch)."""
+        """Advance ``n`` time steps: fused launches of one to eight steps each
+        (one read and one write of the lattice per launch)."""
         if n <= 0:
             return self
         which = ctypes.c_int(0)
@@ -357,9 +357,13 @@ class Lattice:
         torch.cuda.current_stream(self.device).synchronize()
         cur = self._cur
         # an odd number of launches of several steps each would leave the
-        # state in the other buffer: the last one is then split in two
-        last = 4 if n % 4 == 0 and self._max_steps_per_launch() == 4 else 2
-        for parts in ((n,), (n - last, last // 2, last // 2)):
+        # state in the other buffer: one of them is then split in two
+        most = self._max_steps_per_launch()
+        plans = [(n,)]
+        for t in (-(-n // -(-n // most)), n % most or most, 2):
+            if 2 <= t <= n:
+                plans.append((n - t, t // 2, t - t // 2))
+        for parts in plans + [(1,) * n]:
             s = torch.cuda.Stream(device=self.device)
             s.wait_stream(torch.cuda.current_stream(self.device))
             g = torch.cuda.CUDAGraph()

@@ -7,7 +7,8 @@ one strip and several, strips that end inside a warp, within one vector of a
 strip's edge and (4-byte codes) inside a vector, one row per chunk and many,
 the smallest lattice of each number of steps per launch in both directions."""
 
-import numpy as np
+import ctypes
+
 import pytest
 import torch
 
@@ -44,7 +45,7 @@ def same(nx, ny, storage, boundary, steps, cuda, rounding="nearest"):
     assert torch.equal(a, b)
 
 
-TWO = [(8, 256), (128, 16), (17, 120), (33, 121), (40, 124), (19, 241), (64, 1023), (300, 130), (9, 363)]
+TWO = [(8, 125000), (62504, 16), (1000, 1000), (8180, 120), (7900, 124)]
 FOUR = [(8, 187504), (93760, 16), (93751, 17), (8, 187501), (1230, 1240), (1237, 1283)]
 
 
@@ -58,8 +59,8 @@ def test_march_4_byte_codes_equal_single_steps(two_step, cuda, storage, boundary
 @pytest.mark.parametrize("storage", ["f16dev", "bf16dev"])
 @pytest.mark.parametrize("rounding", ["nearest", "stochastic"])
 @pytest.mark.parametrize("boundary", ["cavity", "cavity-ladd", "periodic"])
-@pytest.mark.parametrize("size,steps", [((8, 256), (5,)), ((128, 16), (5,)), ((33, 240), (5,)), ((20, 248), (5,)),
-                                        ((70, 728), (5,)), ((8, 187504), (4, 11)), ((93760, 16), (11,)),
+@pytest.mark.parametrize("size,steps", [((8, 140000), (5,)), ((70000, 16), (5,)), ((4700, 240), (5,)),
+                                        ((4500, 248), (5,)), ((8, 187504), (4, 11)), ((93760, 16), (11,)),
                                         ((1237, 1288), (4, 7))])
 def test_march_16_bit_codes_equal_single_steps(two_step, cuda, storage, rounding, boundary, size, steps):
     same(*size, storage, boundary, steps, cuda, rounding)
@@ -67,7 +68,7 @@ def test_march_16_bit_codes_equal_single_steps(two_step, cuda, storage, rounding
 
 def test_march_unaligned_buffers(two_step, cuda):
     """Buffers that start on 4 bytes only take the element-by-element form."""
-    nx, ny = 24, 256
+    nx, ny = 1500, 1024
     out = []
     for off in (0, 1):
         for several in (1, 0):
@@ -76,13 +77,13 @@ def test_march_unaligned_buffers(two_step, cuda):
             a, b = (s[off:off + 9 * nx * ny].view(9, nx, ny) for s in store)
             g = torch.Generator(device=cuda).manual_seed(1)
             a.copy_(0.1 + 0.01 * torch.rand(9, nx, ny, generator=g, device=cuda))
+            which = ctypes.c_int(-1)
             _lib.call("lbgb_run_fused", a.data_ptr(), b.data_ptr(), nx, ny, _lib.CAVITY, 1.3, 0.05, _lib.F32, 6,
-                      None, torch.cuda.current_stream().cuda_stream)
+                      ctypes.byref(which), torch.cuda.current_stream().cuda_stream)
             torch.cuda.synchronize()
-            out.append((b if several else a).clone())
+            out.append((a, b)[which.value].clone())
             assert float(store[0][:off].abs().sum() + store[0][off + 9 * nx * ny:].abs().sum()) == 0.0
             assert float(store[1][:off].abs().sum() + store[1][off + 9 * nx * ny:].abs().sum()) == 0.0
-    # six steps: three launches end in b, six in a
     assert all(torch.equal(out[0], o) for o in out[1:])
 
 
@@ -90,12 +91,11 @@ def test_march_under_capture_and_max_steps(two_step, cuda):
     _lib.set_tuning(_lib.TUNE_TWO_STEP, 1)
     code = _lib.load().lbgb_max_steps_per_launch
     assert code(4096, 4096, _lib.CAVITY, _lib.F32) == 4
-    assert code(256, 256, _lib.CAVITY_LADD, _lib.F16DEV) == 2
-    assert code(256, 251, _lib.CAVITY_LADD, _lib.F16DEV) == 1
+    assert code(1024, 1032, _lib.CAVITY, _lib.F32) == 2
     assert code(4096, 4096, _lib.CAVITY, _lib.F64) == 1
-    assert code(4, 4, _lib.CAVITY, _lib.F32) == 1
-    lat = PyLB.Lattice(64, 250, 1.2, u0=0.05, device=cuda)
-    ref = PyLB.Lattice(64, 250, 1.2, u0=0.05, device=cuda)
+    assert code(1, 1, _lib.PERIODIC, _lib.F32) == 1
+    lat = PyLB.Lattice(1024, 1000, 1.2, u0=0.05, device=cuda)
+    ref = PyLB.Lattice(1024, 1000, 1.2, u0=0.05, device=cuda)
     replay = lat.capture(6)
     replay()
     replay()
