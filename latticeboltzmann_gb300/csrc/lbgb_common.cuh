@@ -110,7 +110,7 @@ __device__ __forceinline__ void fma16x2(uint32_t a2, unsigned short b, float c_l
 }
 
 // The 16-bit codecs are DEV codecs too: the kernels work on h = f - w_i, the
-// collision in deviation form (collide_dev), so that no population is ever
+// collision in deviation form (relax_dev), so that no population is ever
 // rebuilt from its weight and every rounding acts on a small number.
 template <> struct Codec<LBGB_F16DEV> {
     using raw = unsigned short;
@@ -573,47 +573,137 @@ __device__ __forceinline__ void bgk_collide_native(R (&f)[9], R omega) {
 // stored values.  In the CPU emulation of this arithmetic the 64^2 cavity is
 // at 9e-8 after 1000 and 2000 steps, the storage floor.  Same equilibrium as
 // w_i rho (1 + 3 c.u + 4.5 (c.u)^2 - 1.5 u^2) (c/d2q9.h:59-81) in exact
-// arithmetic.  REST = false leaves h_0 to the caller, which writes it from
-// the rounded stored values.  LOG2K: the values are h 2^LOG2K (FP16 storage
+// arithmetic; 16-bit storage writes it from the rounded stored values.  LOG2K:
+// the values are h 2^LOG2K (FP16 storage
 // keeps its deviations scaled by 2^14; a kernel that collides in those units
 // skips a scaling per value on decode and encode).  Every operation commutes
 // exactly with the power-of-two scale, so the results are bit for bit the
-// unscaled ones times 2^LOG2K.  Returns D (in the same units).
-template <bool REST = true, int LOG2K = 0>
-__device__ __forceinline__ float collide_dev(float (&h)[9], float omega) {
+// unscaled ones times 2^LOG2K.
+//
+// The node's values come one at a time (V = float) or as packed pairs (V =
+// f32x2, two nodes per instruction on sm_100 and later); every operation is
+// rounded on its own or is one FMA as written, so both give the same bits.
+struct f32x2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pk2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void up2(f32x2 a, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vrcp(float a) { return recip_approx(a); }
+__device__ __forceinline__ f32x2 vadd(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 vsub(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 vmul(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 vfma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 vrcp(f32x2 a) {
+    float lo, hi;
+    up2(a, lo, hi);
+    return pk2(recip_approx(lo), recip_approx(hi));
+}
+template <class V> __device__ __forceinline__ V vbc(float x);
+template <> __device__ __forceinline__ float vbc<float>(float x) { return x; }
+template <> __device__ __forceinline__ f32x2 vbc<f32x2>(float x) { return pk2(x, x); }
+
+// Twice the relaxation amounts of the eight moving channels, r[i] = 2 (g +/- d)
+// (the factor takes two halvings out of the sums; powers of two are exact), and
+// the mass deviation D.  The caller applies h_i += (omega / 2) r_i.  No product
+// goes straight into an addition: packed, ptxas fuses the two even with their
+// roundings written out (a multiplication followed by a subtraction gave other
+// bits than the scalar form).  The packed FP32 pipe bounds k_march, so
+// operations are time: 44 here, 94 in all for a FP32 node, 70 for f32dev.
+template <class V, int LOG2K>
+__device__ __forceinline__ V relax_amounts(const V (&h)[9], V (&r)[9]) {
     constexpr float UNIT = 1.f / (float)(1u << LOG2K);
-    const float a13 = h[1] - h[3], b13 = h[1] + h[3];
-    const float a24 = h[2] - h[4], b24 = h[2] + h[4];
-    const float a57 = h[5] - h[7], b57 = h[5] + h[7];
-    const float a68 = h[6] - h[8], b68 = h[6] + h[8];
-    const float d = (((h[0] + b13) + b24) + b57) + b68;
-    const float jx = (a13 + a57) - a68, jy = (a24 + a57) + a68;
-    const float inv = recip_approx(fmaf(d, UNIT, 1.f)) * UNIT;
-    const float ux = jx * inv, uy = jy * inv;
-    const float base = fmaf(-1.5f, fmaf(jx, ux, jy * uy), d);
-    const float sx = jx + jy, sy = jy - jx;
-    const float g13 = fmaf(-0.5f, b13, (1.f / 9.f) * fmaf(4.5f * jx, ux, base));
-    const float g24 = fmaf(-0.5f, b24, (1.f / 9.f) * fmaf(4.5f * jy, uy, base));
-    const float g57 = fmaf(-0.5f, b57, (1.f / 36.f) * fmaf(4.5f * sx, ux + uy, base));
-    const float g68 = fmaf(-0.5f, b68, (1.f / 36.f) * fmaf(4.5f * sy, uy - ux, base));
-    const float d57 = fmaf(sx, 1.f / 12.f, -0.5f * a57);
-    const float d68 = fmaf(sy, 1.f / 12.f, -0.5f * a68);
-    const float d13 = d68 - d57, d24 = -(d57 + d68);
-    h[1] = fmaf(omega, g13 + d13, h[1]);
-    h[3] = fmaf(omega, g13 - d13, h[3]);
-    h[2] = fmaf(omega, g24 + d24, h[2]);
-    h[4] = fmaf(omega, g24 - d24, h[4]);
-    h[5] = fmaf(omega, g57 + d57, h[5]);
-    h[7] = fmaf(omega, g57 - d57, h[7]);
-    h[6] = fmaf(omega, g68 + d68, h[6]);
-    h[8] = fmaf(omega, g68 - d68, h[8]);
-    if constexpr (REST) {
-        float rest = d;
-#pragma unroll
-        for (int i = 1; i < 9; ++i) rest -= h[i];
-        h[0] = rest;
-    }
+    const V a13 = vsub(h[1], h[3]), b13 = vadd(h[1], h[3]);
+    const V a24 = vsub(h[2], h[4]), b24 = vadd(h[2], h[4]);
+    const V n57 = vsub(h[7], h[5]), b57 = vadd(h[5], h[7]);  // -a57
+    const V n68 = vsub(h[8], h[6]), b68 = vadd(h[6], h[8]);  // -a68
+    const V d = vadd(vadd(vadd(vadd(h[0], b13), b24), b57), b68);
+    const V jx = vadd(vsub(a13, n57), n68), jy = vsub(vsub(a24, n57), n68);
+    V inv = vrcp(LOG2K ? vfma(d, vbc<V>(UNIT), vbc<V>(1.f)) : vadd(d, vbc<V>(1.f)));
+    if (LOG2K) inv = vmul(inv, vbc<V>(UNIT));
+    const V ux = vmul(jx, inv), uy = vmul(jy, inv), sx = vadd(jx, jy), sy = vsub(jy, jx);
+    const V base = vfma(vbc<V>(-1.5f), vfma(jx, ux, vmul(jy, uy)), d);
+    const V c45 = vbc<V>(4.5f), w1 = vbc<V>(2.f / 9.f), w5 = vbc<V>(2.f / 36.f), m1 = vbc<V>(-1.f);
+    const V g13 = vfma(m1, b13, vmul(w1, vfma(vmul(c45, jx), ux, base)));
+    const V g24 = vfma(m1, b24, vmul(w1, vfma(vmul(c45, jy), uy, base)));
+    const V g57 = vfma(m1, b57, vmul(w5, vfma(vmul(c45, sx), vadd(ux, uy), base)));
+    const V g68 = vfma(m1, b68, vmul(w5, vfma(vmul(c45, sy), vsub(uy, ux), base)));
+    const V sixth = vbc<V>(2.f / 12.f);
+    const V d57 = vfma(sx, sixth, n57), d68 = vfma(sy, sixth, n68);
+    const V d13 = vsub(d68, d57), m24 = vadd(d57, d68);  // d24 = -m24
+    r[1] = vadd(g13, d13);
+    r[3] = vsub(g13, d13);
+    r[2] = vsub(g24, m24);
+    r[4] = vadd(g24, m24);
+    r[5] = vadd(g57, d57);
+    r[7] = vsub(g57, d57);
+    r[6] = vadd(g68, d68);
+    r[8] = vsub(g68, d68);
     return d;
+}
+
+// The deviations relaxed in place, h[0] left to the caller; returns D.
+template <int LOG2K = 0, class V>
+__device__ __forceinline__ V relax_dev(V (&h)[9], V omega) {
+    V r[9];
+    const V d = relax_amounts<V, LOG2K>(h, r), w = vmul(omega, vbc<V>(0.5f));
+#pragma unroll
+    for (int i = 1; i < 9; ++i) h[i] = vfma(w, r[i], h[i]);
+    return d;
+}
+
+// FP32 populations f collide as deviations too: h = f - w (w as stored by the
+// rest state, so the rest state stays a fixed point), f' = h' + w; the rest
+// population takes what the others lost.  The populations' own rounding is then
+// the only systematic error left.
+template <class V>
+__device__ __forceinline__ void collide_f32(V (&f)[9], V omega) {
+    V h[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) h[i] = vsub(f[i], vbc<V>(wgt<float>(i)));
+    relax_dev(h, omega);
+    V lost = h[0];
+#pragma unroll
+    for (int i = 1; i < 9; ++i) {
+        const V n = vadd(h[i], vbc<V>(wgt<float>(i)));
+        lost = i == 1 ? vsub(f[i], n) : vadd(lost, vsub(f[i], n));
+        f[i] = n;
+    }
+    f[0] = vadd(f[0], lost);
+}
+
+// FP32 deviations: h_0 = D minus the moving ones, D being conserved.
+template <class V>
+__device__ __forceinline__ void collide_f32dev(V (&h)[9], V omega) {
+    V rest = relax_dev(h, omega);
+#pragma unroll
+    for (int i = 1; i < 9; ++i) rest = vsub(rest, h[i]);
+    h[0] = rest;
 }
 
 // The reference lid's Ladd term ((6 w) rho_lid) u0 (cavity_opt1.py:211-212),
@@ -629,7 +719,7 @@ __device__ __forceinline__ R lid_term(R rho_lid, R u0) {
 // deviations and rho_lid = 1 + s: c + c s with c = (6 w) u0 rounded once, so
 // that the low bits of s are not lost in a rounding of 1 + s (which would
 // repeat itself at every lid node and step).
-// With the deviations in units of 2^-LOG2K (see collide_dev) the term is
+// With the deviations in units of 2^-LOG2K (see relax_amounts) the term is
 // c s + c 2^LOG2K, the same value in those units.
 template <int LOG2K = 0>
 __device__ __forceinline__ float lid_term_dev(float s, float u0) {
@@ -704,26 +794,11 @@ __device__ __forceinline__ void collide_encode(typename Codec<DT>::real (&f)[9],
     using C = Codec<DT>;
     using real = typename C::real;
     if constexpr (DT == LBGB_F32) {
-        // FP32 populations collide in the deviation pair form too: h = f - w
-        // (w as stored by the rest state, so the rest state stays a fixed
-        // point), collide_dev, f' = h' + w; the populations' own rounding is
-        // then the only systematic error left
-        real h[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) h[i] = f[i] - wgt<float>(i);
-        collide_dev<false>(h, omega);
-        real d = 0.f;
-#pragma unroll
-        for (int i = 1; i < 9; ++i) {
-            const real fi = h[i] + wgt<float>(i);
-            d += f[i] - fi;
-            f[i] = fi;
-        }
-        f[0] += d;
+        collide_f32(f, omega);
 #pragma unroll
         for (int i = 0; i < 9; ++i) out[i] = f[i];
     } else if constexpr (DT == LBGB_F32DEV) {
-        collide_dev(f, omega);
+        collide_f32dev(f, omega);
 #pragma unroll
         for (int i = 0; i < 9; ++i) out[i] = f[i];
     } else if constexpr (DT == LBGB_F16DEV) {
@@ -731,7 +806,7 @@ __device__ __forceinline__ void collide_encode(typename Codec<DT>::real (&f)[9],
         // mass deviation D S minus what the other eight stored values carry,
         // so the node keeps its mass up to the rounding of h_0 alone.  The
         // pipelined kernel does the same operations.
-        real dms = collide_dev<false>(f, omega) * F16_SCALE;
+        real dms = relax_dev(f, omega) * F16_SCALE;
 #pragma unroll
         for (int i = 1; i < 9; ++i) {
             out[i] = C::enc_h(f[i]);
@@ -739,7 +814,7 @@ __device__ __forceinline__ void collide_encode(typename Codec<DT>::real (&f)[9],
         }
         out[0] = __half_as_ushort(__float2half_rn(dms));
     } else if constexpr (DT == LBGB_BF16DEV) {
-        real dm = collide_dev<false>(f, omega);
+        real dm = relax_dev(f, omega);
 #pragma unroll
         for (int i = 1; i < 9; ++i) {
             out[i] = C::enc_h(f[i]);
@@ -762,7 +837,7 @@ __device__ __forceinline__ void collide_encode(typename Codec<DT>::real (&f)[9],
 template <int DT>
 __device__ __forceinline__ void collide_encode_sr(float (&f)[9], float omega, unsigned short (&out)[9], uint32_t key,
                                                   uint32_t cell) {
-    float dm = collide_dev<false>(f, omega);
+    float dm = relax_dev(f, omega);
     const uint32_t base = sr_pair_base(key, cell & ~1u);
     const bool odd = (cell & 1u) != 0u;
     // the cell's own lane of the pair's word, as the packet kernels round it

@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_mar
     M.iters = K.X1 - K.X0 + 2 * (T - 1);
     M.in = reinterpret_cast<uint4 *>(march_smem + wid * march_smem_warp<T>()) + lane;
     M.delay = M.in + 9 * 32;
-    M.omega = bc2(A.omega);
+    M.omega = vbc<f32x2>(A.omega);
     M.u0 = A.u0;
     if (RAG) {
         const int c0 = __shfl_sync(0xffffffffu, K.c, 0);

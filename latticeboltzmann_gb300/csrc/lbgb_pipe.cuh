@@ -353,7 +353,7 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
                     real h[9];
 #pragma unroll
                     for (int i = 0; i < 9; ++i) h[i] = v[i][j];
-                    hs[0][j] = collide_dev<false, LOG2K>(h, omega);
+                    hs[0][j] = relax_dev<LOG2K>(h, omega);
 #pragma unroll
                     for (int i = 1; i < 9; ++i) hs[i][j] = h[i];
                 }
@@ -384,7 +384,7 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
                 real h[9];
 #pragma unroll
                 for (int i = 0; i < 9; ++i) h[i] = v[i][j];
-                dm[j] = collide_dev<!keep_mass, LOG2K>(h, omega);
+                dm[j] = relax_dev<LOG2K>(h, omega);
 #pragma unroll
                 for (int i = 0; i < 9; ++i) hpost[i][j] = (sr && !UNITS) ? sr_dev<DT>(h[i]) : h[i];
             }

@@ -150,7 +150,7 @@ __device__ __forceinline__ void tile_collide2(const float (&a)[9], const float (
 #pragma unroll
     for (int i = 0; i < 9; ++i) x[i] = pk2(a[i], b[i]);
     uint32_t o[9][2];
-    collide_encode2<DT, false>(x, bc2(omega), 0u, o);
+    collide_encode2<DT, false>(x, vbc<f32x2>(omega), 0u, o);
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
         if constexpr (sizeof(typename Codec<DT>::raw) == 4) {
