@@ -270,6 +270,28 @@ LBGB_API int lbgb_batch_step(const void *src, void *dst, long long total_elems,
                              long long n_tasks, int rows_per_task, int boundary, int dtype,
                              int threads, int blocks, int flat, void *stream);
 
+/* Several steps of a batch per launch, bit for bit those of lbgb_batch_step.
+ * lbgb_batch_plan (host only) says how: *kind, the most steps of one launch
+ * (*most, 1 to 8) and the tasks of a launch of `steps` steps (0: of *most) over
+ * the n instances of sizes nx[b] x ny[b]: *n_tasks entries of four ints, of
+ * which min(capacity, *n_tasks) are written to tasks (host memory).
+ *   LBGB_BATCH_SINGLE  one step per launch only (lbgb_batch_step)
+ *   LBGB_BATCH_MARCH   4 or 2 steps: large batches of 4-byte codes, every
+ *                      instance at least 8 x 16
+ *   LBGB_BATCH_TILE    1 to *most steps: small batches, every instance at least
+ *                      2 x 2
+ * lbgb_batch_steps runs one launch over those tasks (device copy, 16-byte
+ * aligned; a subset advances the instances whose tasks it holds).  Instances,
+ * src, dst: as lbgb_batch_step.  No counterpart in the reference. */
+#define LBGB_BATCH_SINGLE 0
+#define LBGB_BATCH_MARCH 1
+#define LBGB_BATCH_TILE 2
+LBGB_API int lbgb_batch_plan(const int *nx, const int *ny, int n, int boundary, int dtype, int steps, int *kind,
+                             int *most, int *tasks, long long capacity, long long *n_tasks);
+LBGB_API int lbgb_batch_steps(const void *src, void *dst, long long total_elems, const void *instances,
+                              int n_instances, const void *tasks, long long n_tasks, int kind, int steps,
+                              int boundary, int dtype, void *stream);
+
 /* Per-instance amplitude of the shear mode u_x ~ sin(2 pi l / ny):
  * out_dev[b] = 2/(nx ny) sum_{k,l} u_x(k,l) sin(2 pi l / ny), in FP64.
  * The decay diagnostic of shear_wave_opt1.py:174 / shear_wave_decay.py:155-158. */

@@ -66,6 +66,9 @@ SIGNATURES = {
     "lbgb_mass_momentum_noalloc": (_I, [_P, _I64, _I64, _I, _P, _P]),
     "lbgb_convert": (_I, [_P, _I, _I64, _P, _I, _I64, _I64, _P]),
     "lbgb_batch_step": (_I, [_P, _P, ctypes.c_longlong, _P, _I, _P, ctypes.c_longlong, _I, _I, _I, _I, _I, _I, _P]),
+    "lbgb_batch_plan": (_I, [_P, _P, _I, _I, _I, _I, ctypes.POINTER(_I), ctypes.POINTER(_I), _P, ctypes.c_longlong,
+                             ctypes.POINTER(ctypes.c_longlong)]),
+    "lbgb_batch_steps": (_I, [_P, _P, ctypes.c_longlong, _P, _I, _P, ctypes.c_longlong, _I, _I, _I, _I, _P]),
     "lbgb_batch_shear_amplitude": (_I, [_P, ctypes.c_longlong, _P, _I, _I, _P, _P, _P]),
     "lbgb_batch_velocity_change": (_I, [_P, ctypes.c_longlong, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P]),
     "lbgb_row_fft_amplitude": (_I, [_P, _I, _I, _I, _I, _P, _P]),
@@ -99,6 +102,7 @@ SIGNATURES = {
 TUNE_KERNEL, TUNE_STAGES, TUNE_WAIT_LIMIT, TUNE_PIPE_MIN_CELLS, TUNE_TEST_STALL_PRODUCER, TUNE_TWO_STEP = 0, 1, 2, 3, 4, 5
 KERNELS = {"auto": 0, "register": 1, "pipelined": 2}
 NOALLOC_MAX_CELLS = 268435456
+BATCH_SINGLE, BATCH_MARCH, BATCH_TILE = 0, 1, 2
 DIAG_CHUNKS = 64  # LBGB_DIAG_CHUNKS: partials per instance of the batch diagnostics
 
 

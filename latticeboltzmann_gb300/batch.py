@@ -3,10 +3,12 @@
 The reference runs one lattice per process and repeats a script per
 parameter set (e.g. simulators/serial_shear_wave/Python/shear_wave_opt2.py,
 simulators/simple_flows/shear_wave_decay.py:479-548 loops over omega).  Here
-all instances share one population buffer and one launch per step
-(``lbgb_batch_step``) walks a packed queue of warp tasks; a CUDA graph
-captures many steps, and an autotuner picks cells per lane, rows per task and
-the grid shape for the given set of instances.
+all instances share one population buffer, and a launch
+walks a packed queue of tasks.  A launch advances several steps where it can
+(``lbgb_batch_steps``: four for large FP32 batches, up to eight for small ones
+of any storage) and one otherwise (``lbgb_batch_step``, whose cells per lane,
+rows per task and grid an autotuner picks for the given set of instances); a
+CUDA graph captures many steps.
 """
 
 import ctypes
@@ -79,6 +81,8 @@ class BatchedLattice:
         n_sm = _sm_count(self.device)
         self.config = {"flat": True, "vector": False, "rows": 2, "threads": 256, "blocks": n_sm * 8}
         self._tasks = {}
+        self._step_plans = {}
+        self._step_tasks = {}
         self._amp = torch.empty(self.n, dtype=torch.float64, device=self.device)
         self._partials = torch.empty(self.n * _lib.DIAG_CHUNKS, dtype=torch.float64, device=self.device)
         self.active = np.ones(self.n, dtype=bool)  # instances that still advance
@@ -211,6 +215,7 @@ class BatchedLattice:
             self._slice(int(b), other).copy_(self._slice(int(b)))
         self.active = mask
         self._tasks = {k: v for k, v in self._tasks.items() if k[3] is None}
+        self._step_tasks = {k: v for k, v in self._step_tasks.items() if k[1] is None}
 
     def _queue(self, cfg):
         flat = bool(cfg.get("flat", False))
@@ -234,9 +239,65 @@ class BatchedLattice:
                   self.n, tasks.data_ptr(), tasks.shape[0], cfg["rows"], self.bcode, self.code, cfg["threads"],
                   cfg["blocks"], int(flat), self._stream())
 
+    # ------------------------------------------------------------ several steps per launch
+    def _plan(self, steps=0):
+        """(kind, most steps of a launch, host task list of a launch of ``steps`` steps) of lbgb_batch_plan."""
+        nx = np.ascontiguousarray(self._table_np["nx"])
+        ny = np.ascontiguousarray(self._table_np["ny"])
+        kind, most, count = ctypes.c_int(0), ctypes.c_int(1), ctypes.c_longlong(0)
+        tasks = np.zeros((0, 4), dtype=np.int32)
+        while True:
+            _lib.call("lbgb_batch_plan", nx.ctypes.data, ny.ctypes.data, self.n, self.bcode, self.code, int(steps),
+                      ctypes.byref(kind), ctypes.byref(most), tasks.ctypes.data if len(tasks) else None, len(tasks),
+                      ctypes.byref(count))
+            if len(tasks) == count.value:
+                return kind.value, most.value, tasks
+            tasks = np.zeros((count.value, 4), dtype=np.int32)
+
+    def _several(self):
+        key = int(_lib.get_tuning(_lib.TUNE_TWO_STEP))
+        if key not in self._step_plans:
+            self._step_plans[key] = self._plan()[:2]
+        return self._step_plans[key]
+
+    def _launch_steps(self, kind, t):
+        """One launch of t steps of the active instances."""
+        full = self._step_tasks.get((t, None))
+        if full is None:
+            full = self._step_tasks[(t, None)] = torch.from_numpy(self._plan(t)[2]).to(self.device)
+        tasks = full
+        if not self.active.all():
+            key = (t, self.active.tobytes())
+            tasks = self._step_tasks.get(key)
+            if tasks is None:
+                keep = torch.from_numpy(self.active).to(self.device)[full[:, 0].long()]
+                tasks = self._step_tasks[key] = full[keep].contiguous()
+        src, dst = self._buf[self._cur], self._buf[1 - self._cur]
+        if tasks.shape[0] == 0:
+            dst.copy_(src)
+        else:
+            _lib.call("lbgb_batch_steps", src.data_ptr(), dst.data_ptr(), self.total, self._table(True).data_ptr(),
+                      self.n, tasks.data_ptr(), tasks.shape[0], kind, t, self.bcode, self.code, self._stream())
+        self._cur = 1 - self._cur
+
     def step(self, n=1, config=None):
+        """Advance the active instances n steps: several per launch (see
+        lbgb_batch_plan; the same results bit for bit), or one per launch of
+        ``config`` where one is given or several do not apply."""
+        left = int(n)
+        if config is None:
+            kind, most = self._several()
+            while left > 0 and kind != _lib.BATCH_SINGLE:
+                if kind == _lib.BATCH_TILE:
+                    t = -(-left // -(-left // most))
+                else:
+                    t = 4 if left >= 4 else 2
+                    if left < t:
+                        break
+                self._launch_steps(kind, t)
+                left -= t
         cfg = config or self.config
-        for _ in range(int(n)):
+        for _ in range(left):
             self._launch(self._buf[self._cur], self._buf[1 - self._cur], cfg)
             self._cur = 1 - self._cur
         self.steps_taken += int(n)
@@ -248,20 +309,35 @@ class BatchedLattice:
             raise ValueError("capture: n must be a positive even number")
         self.task_queue(self.config["vector"], self.config["rows"], self.config.get("flat", False))  # outside the capture
         self._table(self.config["vector"])
-        # load the kernel outside the capture: two steps on a copy of the state
+        # an odd number of launches would leave the state in the other buffer:
+        # one of them is then split in two
+        _, most = self._several()
+        plans = [(n,)]
+        for t in (-(-n // -(-n // most)), n % most or most, 2):
+            if 2 <= t <= n:
+                plans.append((n - t, t // 2, t - t // 2))
         saved = self.state.clone()
         cur, taken = self._cur, self.steps_taken
-        self.step(2)
-        self._buf[cur].copy_(saved)
-        self._cur, self.steps_taken = cur, taken
+        # the first split whose launches return to this buffer, run once outside
+        # the capture (kernels loaded, task lists on the device)
+        for parts in plans:
+            for p in parts:
+                self.step(p)
+            back = self._cur == cur
+            self._buf[cur].copy_(saved)
+            self._cur, self.steps_taken = cur, taken
+            if back:
+                break
+        else:
+            raise RuntimeError("capture: no even number of launches for %d steps" % n)
         torch.cuda.synchronize(self.device)
         s = torch.cuda.Stream(device=self.device)
         s.wait_stream(torch.cuda.current_stream(self.device))
         g = torch.cuda.CUDAGraph()
-        cur, taken = self._cur, self.steps_taken
         with torch.cuda.stream(s):
             with torch.cuda.graph(g, stream=s):
-                self.step(n)
+                for p in parts:
+                    self.step(p)
         self._cur, self.steps_taken = cur, taken
         torch.cuda.current_stream(self.device).wait_stream(s)
         batch = self

@@ -16,16 +16,12 @@
 // dereferenced.
 #pragma once
 
-namespace lbgb {
+#include <algorithm>
+#include <vector>
 
-struct BatchInstanceDev {
-    long long offset;
-    int nx, ny;
-    double omega, u0;
-    int vec;
-    unsigned int cell_base;
-};
-static_assert(sizeof(BatchInstanceDev) == sizeof(lbgb_batch_instance), "instance table layout");
+#include "lbgb_batch.h"
+
+namespace lbgb {
 
 template <int DT, int BC, int VW>
 __global__ void __launch_bounds__(256)
@@ -214,6 +210,9 @@ __global__ void k_batch_amplitude_finish(const BatchInstanceDev *__restrict__ in
     const long long n = (long long)in.nx * in.ny;
     const bool ok = in.nx > 0 && in.ny > 0 && in.offset >= 0 && in.offset + 9 * n <= total_elems;
     double s = 0.0;
+    // in chunk order, sixteen loads at a time (one by one the 64 round trips to
+    // the L2 took 6 us)
+#pragma unroll 16
     for (int c = 0; c < LBGB_DIAG_CHUNKS; ++c) s += part[(long long)b * LBGB_DIAG_CHUNKS + c];
     out[b] = ok ? s * 2.0 / (double)n : 0.0;
 }
@@ -269,6 +268,7 @@ __global__ void k_batch_change_finish(int n_inst, const double *__restrict__ par
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= n_inst) return;
     double m = part[(long long)b * LBGB_DIAG_CHUNKS];
+#pragma unroll 16
     for (int c = 1; c < LBGB_DIAG_CHUNKS; ++c) m = fmax(m, part[(long long)b * LBGB_DIAG_CHUNKS + c]);
     out[b] = (float)m;
 }
@@ -443,4 +443,207 @@ extern "C" int lbgb_batch_velocity_change(const void *f, long long total_elems, 
     if (rc) return rc;
     k_batch_change_finish<<<(n_instances + 127) / 128, 128, 0, s>>>(n_instances, partials, out_dev);
     return check_launch("k_batch_change_finish");
+}
+
+namespace lbgb {
+
+// Lanes that write a strip of `left` columns at the lowest cost, and the lanes
+// of the strip itself: 32, 16 or 8, two of which only feed their neighbours.
+static int batch_lanes(int left, int *first) {
+    static const int kinds[] = {32, 16, 8};
+    if (left <= 0) return 0;
+    if (left > 4096) {
+        *first = 32;
+        return 32 + batch_lanes(left - 120, first);
+    }
+    thread_local std::vector<int> cost, kind;
+    if (cost.empty()) cost.push_back(0), kind.push_back(0);
+    for (int c = (int)cost.size(); c <= left; ++c) {
+        int best = 0, k = 0;
+        for (int g : kinds) {
+            const int rest = c - 4 * (g - 2), n = g + (rest > 0 ? cost[rest] : 0);
+            if (!k || n < best) best = n, k = g;
+        }
+        cost.push_back(best);
+        kind.push_back(k);
+    }
+    *first = kind[left];
+    return cost[left];
+}
+
+struct BatchTask {
+    int x, y, z, w;
+};
+
+// March: chunks of `target` rows of every strip.
+static void batch_march_tasks(const int *nx, const int *ny, int n, bool walls, int T, int target,
+                              std::vector<BatchTask> &out) {
+    out.clear();
+    for (int b = 0; b < n; ++b) {
+        const int most = std::max(1, std::min(target, nx[b] - T));
+        for (int y = 0; y < ny[b];) {
+            int g = 32;
+            if (!walls) batch_lanes(ny[b] - y, &g);
+            const int groups = 32 / g;
+            int chunks = (nx[b] + most - 1) / most;
+            chunks = (chunks + groups - 1) / groups * groups;
+            int rows = (nx[b] + chunks - 1) / chunks;
+            for (int x = 0; x < nx[b]; x += rows * groups) out.push_back({b, x, y, rows | (g << 16)});
+            y += 4 * (g - 2);
+        }
+    }
+}
+
+// Tiles of T steps; each instance's shape for its share of the SMs.  Returns
+// the expected cycles per step, or 0 where an instance has no tile.
+static double batch_tile_tasks(const int *nx, const int *ny, int n, int T, int element, double cell, int sms,
+                               std::vector<BatchTask> &out) {
+    out.clear();
+    double all = 0.0, work = 0.0;
+    for (int b = 0; b < n; ++b) all += (double)nx[b] * ny[b];
+    for (int b = 0; b < n; ++b) {
+        const double share = sms * ((double)nx[b] * ny[b] / all);
+        const int m = share < 1.0 ? 1 : (int)(share + 0.5);
+        if (T > nx[b] || T > ny[b]) return 0.0;
+        const TileShape t = tile_shape(nx[b], ny[b], T, element, cell, m);
+        if (!t.rows || t.rows > 0xffff) return 0.0;
+        const int co = std::min(t.cols, ny[b]);
+        for (int x = 0; x < nx[b]; x += t.rows)
+            for (int y = 0; y < ny[b]; y += co) {
+                const int ro = std::min(t.rows, nx[b] - x), c = std::min(co, ny[b] - y);
+                out.push_back({b, x, y, ro | (c << 16)});
+            }
+        // one instance on m SMs
+        work += tile_cost(nx[b], ny[b], t, cell, m) * T * m;
+    }
+    return work / sms / T;
+}
+
+}  // namespace lbgb
+
+extern "C" int lbgb_batch_plan(const int *nx, const int *ny, int n, int boundary, int dtype, int steps, int *kind,
+                               int *most, int *tasks, long long capacity, long long *n_tasks) {
+    using namespace lbgb;
+    if (!nx || !ny || n <= 0 || !kind || !most || !n_tasks || steps < 0 || (capacity > 0 && !tasks)) {
+        set_error("lbgb_batch_plan: null argument or empty batch");
+        return LBGB_EINVAL;
+    }
+    if (raw_size(dtype) == 0) {
+        set_error("lbgb_batch_plan: unsupported storage code %d", dtype);
+        return LBGB_EDTYPE;
+    }
+    if (boundary != LBGB_PERIODIC && boundary != LBGB_CAVITY && boundary != LBGB_CAVITY_LADD) {
+        set_error("lbgb_batch_plan: unknown boundary code %d", boundary);
+        return LBGB_EINVAL;
+    }
+    const int es = (int)raw_size(dtype), sms = sm_count();
+    const bool walls = boundary != LBGB_PERIODIC;
+    double cells = 0.0;
+    bool march = es == 4, tile = true;
+    for (int b = 0; b < n; ++b) {
+        if (nx[b] <= 0 || ny[b] <= 0) {
+            set_error("lbgb_batch_plan: instance %d has size %d x %d", b, nx[b], ny[b]);
+            return LBGB_EINVAL;
+        }
+        cells += (double)nx[b] * ny[b];
+        march = march && nx[b] >= 8 && ny[b] >= 16;
+        tile = tile && nx[b] >= 2 && ny[b] >= 2 && ny[b] <= 0x7fff;
+    }
+    *kind = LBGB_BATCH_SINGLE;
+    *most = 1;
+    *n_tasks = 0;
+    if (!g_tune.two_step) return LBGB_OK;
+    std::vector<BatchTask> list;
+    // the march for large batches of 4-byte codes, tiles for small ones
+    const double tile_most = dtype == LBGB_F64 ? 150000 : 1200000;
+    if (march && cells > tile_most) {
+        *kind = LBGB_BATCH_MARCH;
+        *most = 4;
+        const int T = steps == 2 ? 2 : 4;
+        // rows of a chunk: as march_chunks, over the warps of the whole batch
+        static const int targets[] = {4, 8, 12, 16, 24, 32, 48, 64, 96, 128};
+        double least = 0.0;
+        int best = 4;
+        for (int r : targets) {
+            double warps = 0.0;
+            batch_march_tasks(nx, ny, n, walls, T, r, list);
+            warps = (double)list.size();
+            const double load = warps / (4.0 * sms), cost = (r + 2 * T - 1) * ((load > 1.9 ? load : 1.9) + 1.0);
+            if (least == 0.0 || cost < least) least = cost, best = r;
+        }
+        batch_march_tasks(nx, ny, n, walls, T, best, list);
+        // the longest chunks first
+        std::stable_sort(list.begin(), list.end(),
+                         [](const BatchTask &a, const BatchTask &c) { return (a.w & 0xffff) > (c.w & 0xffff); });
+    } else if (tile && cells <= tile_most) {
+        const double cell = dtype == LBGB_F64 ? 13.5 : 1.45;
+        double least = 0.0;
+        int best = 0;
+        for (int T = 2; T <= TILE_MAX_STEPS; ++T) {
+            const double c = batch_tile_tasks(nx, ny, n, T, es, cell, sms, list);
+            if (c > 0.0 && (!best || c < least)) least = c, best = T;
+        }
+        if (best < 2) return LBGB_OK;
+        *kind = LBGB_BATCH_TILE;
+        *most = best;
+        const int T = steps >= 1 && steps < best ? steps : best;
+        if (batch_tile_tasks(nx, ny, n, T, es, cell, sms, list) == 0.0) return LBGB_OK;
+    } else {
+        return LBGB_OK;
+    }
+    if (list.size() > 0x7fffffffull) {
+        set_error("lbgb_batch_plan: too many tasks");
+        return LBGB_EINVAL;
+    }
+    *n_tasks = (long long)list.size();
+    const long long m = std::min<long long>(capacity, *n_tasks);
+    if (m > 0) memcpy(tasks, list.data(), (size_t)m * sizeof(BatchTask));
+    return LBGB_OK;
+}
+
+extern "C" int lbgb_batch_steps(const void *src, void *dst, long long total_elems, const void *instances,
+                                int n_instances, const void *tasks, long long n_tasks, int kind, int steps,
+                                int boundary, int dtype, void *stream) {
+    using namespace lbgb;
+    if (raw_size(dtype) == 0) {
+        set_error("lbgb_batch_steps: unsupported storage code %d", dtype);
+        return LBGB_EDTYPE;
+    }
+    if (!src || !dst || !instances || !tasks || n_instances <= 0 || n_tasks < 0 || n_tasks > 0x7fffffffll ||
+        total_elems <= 0) {
+        set_error("lbgb_batch_steps: null buffer, empty batch or too many tasks");
+        return LBGB_EINVAL;
+    }
+    if (boundary != LBGB_PERIODIC && boundary != LBGB_CAVITY && boundary != LBGB_CAVITY_LADD) {
+        set_error("lbgb_batch_steps: unknown boundary code %d", boundary);
+        return LBGB_EINVAL;
+    }
+    const bool march = kind == LBGB_BATCH_MARCH && (dtype == LBGB_F32 || dtype == LBGB_F32DEV) && (steps == 2 || steps == 4);
+    const bool tile = kind == LBGB_BATCH_TILE && steps >= 1 && steps <= TILE_MAX_STEPS;
+    if (!march && !tile) {
+        set_error("lbgb_batch_steps: kind %d does not take %d steps of storage code %d", kind, steps, dtype);
+        return LBGB_EINVAL;
+    }
+    const size_t bytes = (size_t)total_elems * raw_size(dtype);
+    const char *a = static_cast<const char *>(src), *b = static_cast<const char *>(dst);
+    if (a < b + bytes && b < a + bytes) {
+        set_error("lbgb_batch_steps: src and dst overlap");
+        return LBGB_EINVAL;
+    }
+    if (!aligned(src, 16) || !aligned(dst, 16) || !aligned(instances, 8) || !aligned(tasks, 16)) {
+        set_error("lbgb_batch_steps: buffers must be 16-byte aligned (instance table 8-byte)");
+        return LBGB_EINVAL;
+    }
+    if (n_tasks == 0) return LBGB_OK;
+    const BatchCall c{src,          dst, total_elems, static_cast<const BatchInstanceDev *>(instances),
+                      n_instances,  static_cast<const int4 *>(tasks), (int)n_tasks, boundary, steps};
+    cudaStream_t s = (cudaStream_t)stream;
+    if (march) return dtype == LBGB_F32 ? launch_march_batch<LBGB_F32>(c, s) : launch_march_batch<LBGB_F32DEV>(c, s);
+    switch (dtype) {
+    case LBGB_F32: return launch_tile_batch<LBGB_F32>(c, s);
+    case LBGB_F64: return launch_tile_batch<LBGB_F64>(c, s);
+    case LBGB_F16DEV: return launch_tile_batch<LBGB_F16DEV>(c, s);
+    case LBGB_BF16DEV: return launch_tile_batch<LBGB_BF16DEV>(c, s);
+    default: return launch_tile_batch<LBGB_F32DEV>(c, s);
+    }
 }

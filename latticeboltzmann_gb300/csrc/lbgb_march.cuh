@@ -38,6 +38,7 @@
 // codes gain 6 % from unrolling it.
 #pragma once
 
+#include "lbgb_batch.h"
 #include "lbgb_common.cuh"
 #include "lbgb_march.h"
 #include "lbgb_pair.cuh"
@@ -52,8 +53,8 @@ constexpr int march_smem_warp() { return T * MARCH_ROW; }  // one input row, T -
 // One cell towards higher / lower l: the words of a vector shifted by one
 // element, the missing element from the neighbouring lane.
 template <int ES>
-__device__ __forceinline__ void shift_up(uint32_t (&w)[4]) {
-    const uint32_t p = __shfl_up_sync(0xffffffffu, w[3], 1);
+__device__ __forceinline__ void shift_up(uint32_t (&w)[4], int width) {
+    const uint32_t p = __shfl_up_sync(0xffffffffu, w[3], 1, width);
     if constexpr (ES == 4) {
         w[3] = w[2];
         w[2] = w[1];
@@ -67,8 +68,8 @@ __device__ __forceinline__ void shift_up(uint32_t (&w)[4]) {
     }
 }
 template <int ES>
-__device__ __forceinline__ void shift_down(uint32_t (&w)[4]) {
-    const uint32_t p = __shfl_down_sync(0xffffffffu, w[0], 1);
+__device__ __forceinline__ void shift_down(uint32_t (&w)[4], int width) {
+    const uint32_t p = __shfl_down_sync(0xffffffffu, w[0], 1, width);
     if constexpr (ES == 4) {
         w[0] = w[1];
         w[1] = w[2];
@@ -82,9 +83,9 @@ __device__ __forceinline__ void shift_down(uint32_t (&w)[4]) {
     }
 }
 template <int ES>
-__device__ __forceinline__ void shift_y(int ch, uint32_t (&w)[4]) {
-    if (cy(ch) > 0) shift_up<ES>(w);
-    if (cy(ch) < 0) shift_down<ES>(w);
+__device__ __forceinline__ void shift_y(int ch, uint32_t (&w)[4], int width) {
+    if (cy(ch) > 0) shift_up<ES>(w, width);
+    if (cy(ch) < 0) shift_down<ES>(w, width);
 }
 __device__ __forceinline__ void ld_words(const uint4 *p, uint32_t (&w)[4]) {
     const uint4 q = *p;
@@ -209,15 +210,22 @@ __device__ __forceinline__ void march_collide(const uint32_t (&v)[9][4], f32x2 o
 struct MarchTask {
     int X0, X1, c, nwrite, jt;
     bool bottom, top;
+    int width;  // GROUPS: lanes of a group
+    bool vec;   // GROUPS: rows of whole 16-byte vectors
 };
 
-// RAG: rows of any length and alignment (4-byte codes), element by element.
-template <int DT, int BC, int T, bool SRND, bool RAG>
+// How a strip is read and written: whole 16-byte vectors; element by element
+// (4-byte codes, rows of any length and alignment); or, for the strips of a
+// batch (4-byte codes), either as the instance has it, by groups of 32, 16 or 8
+// lanes that march down chunks of rows of their own.
+enum { MARCH_VECTORS, MARCH_RAGGED, MARCH_GROUPS };
+
+template <int DT, int BC, int T, bool SRND, int MODE>
 struct March {
     using raw = typename Codec<DT>::raw;
     static constexpr int ES = (int)sizeof(raw), NC = 16 / ES;
-    static constexpr bool WALLS = BC != LBGB_PERIODIC;
-    static_assert(!RAG || ES == 4, "element by element: 4-byte codes");
+    static constexpr bool WALLS = BC != LBGB_PERIODIC, RAG = MODE == MARCH_RAGGED, GRP = MODE == MARCH_GROUPS;
+    static_assert(MODE == MARCH_VECTORS || ES == 4, "element by element: 4-byte codes");
 
     const raw *__restrict__ src;
     raw *__restrict__ dst;
@@ -227,14 +235,14 @@ struct March {
     uint4 *in, *delay;  // this lane's vector of [channel] and [step][plane], 32 lanes each
     f32x2 omega;
     float u0;
-    int col[RAG ? 4 : 1];  // RAG: column of cell 32 i + lane of the warp's 128
+    int col[MODE == MARCH_VECTORS ? 1 : 4];  // RAG: columns of cells 32 i + lane of the warp's 128; GRP: of the lane's cells
     uint32_t key[T];
 
     __device__ __forceinline__ int wrap(int r) const { return r < 0 ? r + nx : (r >= nx ? r - nx : r); }
 
     // copies the pulled rows of lattice row r (channel i from row r - cx_i)
     __device__ __forceinline__ void issue(int r) const {
-        const int c = RAG ? 0 : K.c;
+        const int c = RAG || (GRP && !K.vec) ? 0 : K.c;
         const raw *q0 = src + (size_t)wrap(r) * ny + c, *qm = src + (size_t)wrap(r - 1) * ny + c,
                   *qp = src + (size_t)wrap(r + 1) * ny + c;
 #pragma unroll
@@ -244,6 +252,10 @@ struct March {
                 float *s = reinterpret_cast<float *>(in - lane + ch * 32) + lane;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) cp_async4(s + 32 * i, q + col[i]);
+            } else if (GRP && !K.vec) {
+                float *s = reinterpret_cast<float *>(in + ch * 32);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) cp_async4(s + i, q + col[GRP ? i : 0]);
             } else {
                 cp_async16(in + ch * 32, q);
             }
@@ -261,7 +273,7 @@ struct March {
     // the lane's cells of row k, channel ch
     __device__ __forceinline__ void ld_row(int ch, int k, uint32_t (&w)[4]) const {
         const raw *q = src + ch * cs + (size_t)k * ny;
-        if constexpr (RAG) {
+        if constexpr (MODE != MARCH_VECTORS) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) w[j] = raw_bits(ld1(q + (K.c + j) % ny));
         } else {
@@ -274,7 +286,7 @@ struct March {
     // of some step may touch a side wall.
     template <bool EDGE, bool SIDE, int UNROLL>
     __device__ __forceinline__ void row(int it, uint32_t (&eg)[T][3], uint32_t (&seam)[T][2]) const {
-        const int jt = RAG ? K.jt : NC - 1;
+        const int jt = MODE == MARCH_VECTORS ? NC - 1 : K.jt, width = GRP ? K.width : 32;
         int k = wrap(r_first + it);
         uint32_t o[9][4];
         {
@@ -284,7 +296,7 @@ struct March {
 #pragma unroll
             for (int ch = 0; ch < 9; ++ch) ld_words(in + ch * 32, v[ch]);
 #pragma unroll
-            for (int ch = 0; ch < 9; ++ch) shift_y<ES>(ch, v[ch]);
+            for (int ch = 0; ch < 9; ++ch) shift_y<ES>(ch, v[ch], width);
             Lid lid{1.f, 0.f, false, false};
             if constexpr (EDGE) {
                 const uint32_t lc[4] = {cell_code<ES>(v[CE], jt), cell_code<ES>(v[CNE], jt), cell_code<ES>(v[CW], jt),
@@ -340,7 +352,7 @@ struct March {
                 uint4 *dk = dl + (3 + 3 * ((it & 1) ^ 1)) * 32;
                 if constexpr (EDGE) {
                     uint32_t t[4] = {o[CNW][0], o[CNW][1], o[CNW][2], o[CNW][3]};
-                    shift_up<ES>(t);
+                    shift_up<ES>(t, width);
                     lw = cell_code<ES>(o[CW], jt);
                     lnw = cell_code<ES>(t, jt);
                 }
@@ -353,7 +365,7 @@ struct March {
                 }
             }
 #pragma unroll
-            for (int ch = 0; ch < 9; ++ch) shift_y<ES>(ch, o[ch]);
+            for (int ch = 0; ch < 9; ++ch) shift_y<ES>(ch, o[ch], width);
             st_words(dx, o[CE]);
             st_words(dx + 32, o[CNE]);
             st_words(dx + 64, o[CSE]);
@@ -375,14 +387,14 @@ struct March {
             }
             k = r;
         }
-        if (it >= 2 * (T - 1)) {
+        if (it >= 2 * (T - 1) && (!GRP || it - 2 * (T - 1) < K.X1 - K.X0)) {
             raw *q = dst + (size_t)k * ny + K.c;
-            if constexpr (RAG) {
+            if (RAG || (GRP && !K.vec)) {
 #pragma unroll
                 for (int ch = 0; ch < 9; ++ch)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        if (j < K.nwrite) st_cs(reinterpret_cast<unsigned int *>(q + ch * cs + j), o[ch][j]);
+                        if (j < K.nwrite) st_cs(reinterpret_cast<unsigned int *>(q + ch * cs + j * (4 / ES)), o[ch][j]);
             } else if (K.nwrite) {
 #pragma unroll
                 for (int ch = 0; ch < 9; ++ch)
@@ -417,7 +429,7 @@ struct March {
     static constexpr int MAIN_UNROLL = ES == 4 ? T : 1, EDGE_UNROLL = ES == 4 ? T : 1;
 };
 
-template <int DT, int BC, int T, bool SRND, bool RAG>
+template <int DT, int BC, int T, bool SRND, int MODE>
 __global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_march(const MarchArgs A) {
     constexpr int NC = 16 / (int)sizeof(typename Codec<DT>::raw), W = MARCH_LANES * NC;
     constexpr bool WALLS = BC != LBGB_PERIODIC;
@@ -447,7 +459,9 @@ __global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_mar
     const bool edge = WALLS && __any_sync(0xffffffffu, K.bottom || K.top);
     K.c %= A.ny;
     if (K.c < 0) K.c += A.ny;
-    March<DT, BC, T, SRND, RAG> M;
+    K.width = 32;
+    K.vec = MODE == MARCH_VECTORS;
+    March<DT, BC, T, SRND, MODE> M;
     M.src = static_cast<const typename Codec<DT>::raw *>(A.src);
     M.dst = static_cast<typename Codec<DT>::raw *>(A.dst);
     M.nx = A.nx;
@@ -461,10 +475,10 @@ __global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_mar
     M.delay = M.in + 9 * 32;
     M.omega = vbc<f32x2>(A.omega);
     M.u0 = A.u0;
-    if (RAG) {
+    if constexpr (MODE == MARCH_RAGGED) {
         const int c0 = __shfl_sync(0xffffffffu, K.c, 0);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) M.col[RAG ? i : 0] = (c0 + 32 * i + lane) % A.ny;
+        for (int i = 0; i < 4; ++i) M.col[i] = (c0 + 32 * i + lane) % A.ny;
     }
 #pragma unroll
     for (int s = 0; s < T; ++s) M.key[s] = SRND ? sr_step_key(A.sr_seed, *A.sr_step + A.sr_offset + s) : 0u;
@@ -474,7 +488,7 @@ __global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_mar
         M.template run<false>();
 }
 
-template <int DT, int BC, int T, bool SRND, bool RAG>
+template <int DT, int BC, int T, bool SRND, int MODE>
 static int launch_march_v(const MarchCall &c, cudaStream_t s) {
     constexpr int NC = 16 / (int)sizeof(typename Codec<DT>::raw);
     MarchArgs A;
@@ -490,17 +504,17 @@ static int launch_march_v(const MarchCall &c, cudaStream_t s) {
     A.sr_seed = c.sr_seed;
     A.sr_offset = c.sr_offset;
     const long long tasks = (long long)A.nstrips * A.nchunks;
-    k_march<DT, BC, T, SRND, RAG><<<(unsigned)((tasks + MARCH_WPB - 1) / MARCH_WPB), MARCH_WPB * 32,
+    k_march<DT, BC, T, SRND, MODE><<<(unsigned)((tasks + MARCH_WPB - 1) / MARCH_WPB), MARCH_WPB * 32,
                                     MARCH_WPB * march_smem_warp<T>(), s>>>(A);
     return check_launch("k_march");
 }
 
-template <int DT, int T, bool SRND, bool RAG>
+template <int DT, int T, bool SRND, int MODE>
 static int launch_march_bc(const MarchCall &c, cudaStream_t s) {
     switch (c.boundary) {
-    case LBGB_CAVITY: return launch_march_v<DT, LBGB_CAVITY, T, SRND, RAG>(c, s);
-    case LBGB_CAVITY_LADD: return launch_march_v<DT, LBGB_CAVITY_LADD, T, SRND, RAG>(c, s);
-    default: return launch_march_v<DT, LBGB_PERIODIC, T, SRND, RAG>(c, s);
+    case LBGB_CAVITY: return launch_march_v<DT, LBGB_CAVITY, T, SRND, MODE>(c, s);
+    case LBGB_CAVITY_LADD: return launch_march_v<DT, LBGB_CAVITY_LADD, T, SRND, MODE>(c, s);
+    default: return launch_march_v<DT, LBGB_PERIODIC, T, SRND, MODE>(c, s);
     }
 }
 
@@ -508,12 +522,87 @@ template <int DT>
 int launch_march(const MarchCall &c, cudaStream_t s) {
     if constexpr (sizeof(typename Codec<DT>::raw) == 4) {
         if (c.ragged)
-            return c.steps == 4 ? launch_march_bc<DT, 4, false, true>(c, s) : launch_march_bc<DT, 2, false, true>(c, s);
+            return c.steps == 4 ? launch_march_bc<DT, 4, false, MARCH_RAGGED>(c, s) : launch_march_bc<DT, 2, false, MARCH_RAGGED>(c, s);
     } else {
         if (c.sr_step)
-            return c.steps == 4 ? launch_march_bc<DT, 4, true, false>(c, s) : launch_march_bc<DT, 2, true, false>(c, s);
+            return c.steps == 4 ? launch_march_bc<DT, 4, true, MARCH_VECTORS>(c, s) : launch_march_bc<DT, 2, true, MARCH_VECTORS>(c, s);
     }
-    return c.steps == 4 ? launch_march_bc<DT, 4, false, false>(c, s) : launch_march_bc<DT, 2, false, false>(c, s);
+    return c.steps == 4 ? launch_march_bc<DT, 4, false, MARCH_VECTORS>(c, s) : launch_march_bc<DT, 2, false, MARCH_VECTORS>(c, s);
+}
+
+// The march over a batch: a warp takes a task, a strip of one instance.  Entries
+// that do not fit the buffer or the instance are skipped, never dereferenced.
+template <int DT, int BC, int T>
+__global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_march_batch(const BatchCall B) {
+    using raw = typename Codec<DT>::raw;
+    constexpr bool WALLS = BC != LBGB_PERIODIC;
+    extern __shared__ __align__(16) unsigned char march_smem[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int task = blockIdx.x * MARCH_WPB + wid;
+    if (task >= B.n_tasks) return;
+    const int4 tk = B.tasks[task];
+    if (tk.x < 0 || tk.x >= B.n_inst) return;
+    const BatchInstanceDev in = B.inst[tk.x];
+    const long long need = 9ll * in.nx * in.ny;
+    const int rows = tk.w & 0xffff, width = tk.w >> 16;
+    if (in.nx < 8 || in.ny < 16 || in.offset < 0 || in.offset + need > B.total || in.offset % 4 != 0) return;
+    if (tk.y < 0 || tk.y >= in.nx || tk.z < 0 || tk.z >= in.ny || rows < 1 || rows + T > in.nx) return;
+    if (!(width == 32 || (!WALLS && (width == 16 || width == 8)))) return;
+    March<DT, BC, T, false, MARCH_GROUPS> M;
+    M.src = static_cast<const raw *>(B.src) + in.offset;
+    M.dst = static_cast<raw *>(B.dst) + in.offset;
+    M.nx = in.nx;
+    M.ny = in.ny;
+    M.cs = (size_t)in.nx * in.ny;
+    M.lane = lane;
+    MarchTask K;
+    const int gl = lane & (width - 1);
+    K.X0 = tk.y + (lane / width) * rows;
+    const bool some = K.X0 < in.nx;  // groups past the end repeat the first and write nothing
+    if (!some) K.X0 = tk.y;
+    K.X1 = min(K.X0 + rows, in.nx);
+    K.c = tk.z + (gl - 1) * 4;
+    K.nwrite = some && gl >= 1 && gl <= width - 2 ? min(max(in.ny - K.c, 0), 4) : 0;
+    K.bottom = K.c == 0;
+    K.top = K.c < in.ny && K.c + 4 >= in.ny;
+    K.jt = (in.ny - 1) & 3;
+    K.width = width;
+    K.vec = in.ny % 4 == 0;
+    const bool edge = WALLS && __any_sync(0xffffffffu, K.bottom || K.top);
+    K.c %= in.ny;
+    if (K.c < 0) K.c += in.ny;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) M.col[i] = (K.c + i) % in.ny;
+    M.K = K;
+    M.r_first = K.X0 - (T - 1);
+    M.iters = rows + 2 * (T - 1);
+    M.in = reinterpret_cast<uint4 *>(march_smem + wid * march_smem_warp<T>()) + lane;
+    M.delay = M.in + 9 * 32;
+    M.omega = vbc<f32x2>((float)in.omega);
+    M.u0 = (float)in.u0;
+#pragma unroll
+    for (int s = 0; s < T; ++s) M.key[s] = 0u;
+    if (edge)
+        M.template run<WALLS>();
+    else
+        M.template run<false>();
+}
+
+template <int DT, int T>
+static int launch_march_batch_t(const BatchCall &c, cudaStream_t s) {
+    const unsigned grid = (unsigned)((c.n_tasks + MARCH_WPB - 1) / MARCH_WPB);
+    constexpr int smem = MARCH_WPB * march_smem_warp<T>();
+    switch (c.boundary) {
+    case LBGB_CAVITY: k_march_batch<DT, LBGB_CAVITY, T><<<grid, MARCH_WPB * 32, smem, s>>>(c); break;
+    case LBGB_CAVITY_LADD: k_march_batch<DT, LBGB_CAVITY_LADD, T><<<grid, MARCH_WPB * 32, smem, s>>>(c); break;
+    default: k_march_batch<DT, LBGB_PERIODIC, T><<<grid, MARCH_WPB * 32, smem, s>>>(c);
+    }
+    return check_launch("k_march_batch");
+}
+
+template <int DT>
+int launch_march_batch(const BatchCall &c, cudaStream_t s) {
+    return c.steps == 4 ? launch_march_batch_t<DT, 4>(c, s) : launch_march_batch_t<DT, 2>(c, s);
 }
 
 }  // namespace lbgb

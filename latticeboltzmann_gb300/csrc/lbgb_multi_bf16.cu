@@ -4,4 +4,5 @@
 namespace lbgb {
 template int launch_march<LBGB_BF16DEV>(const MarchCall &c, cudaStream_t s);
 template int launch_tile<LBGB_BF16DEV>(const TileCall &c, cudaStream_t s);
+template int launch_tile_batch<LBGB_BF16DEV>(const BatchCall &c, cudaStream_t s);
 }  // namespace lbgb

@@ -4,4 +4,6 @@
 namespace lbgb {
 template int launch_march<LBGB_F32>(const MarchCall &c, cudaStream_t s);
 template int launch_tile<LBGB_F32>(const TileCall &c, cudaStream_t s);
+template int launch_march_batch<LBGB_F32>(const BatchCall &c, cudaStream_t s);
+template int launch_tile_batch<LBGB_F32>(const BatchCall &c, cudaStream_t s);
 }  // namespace lbgb

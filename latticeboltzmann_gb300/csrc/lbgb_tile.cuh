@@ -23,6 +23,7 @@
 // the storage's own codes: the results equal single steps bit for bit.
 #pragma once
 
+#include "lbgb_batch.h"
 #include "lbgb_common.cuh"
 #include "lbgb_pair.cuh"
 #include "lbgb_tile.h"
@@ -316,6 +317,69 @@ int launch_tile(const TileCall &c, cudaStream_t s) {
     case LBGB_CAVITY: return launch_tile_v<DT, LBGB_CAVITY, false>(c, s);
     case LBGB_CAVITY_LADD: return launch_tile_v<DT, LBGB_CAVITY_LADD, false>(c, s);
     default: return launch_tile_v<DT, LBGB_PERIODIC, false>(c, s);
+    }
+}
+
+// Tiles of a batch: a block takes a task, a tile of one instance.  Entries that
+// do not fit the buffer, the instance or a tile are skipped, never dereferenced.
+template <int DT, int BC>
+__global__ void __launch_bounds__(TILE_THREADS, 1) k_tile_batch(const BatchCall B) {
+    using raw = typename Codec<DT>::raw;
+    extern __shared__ __align__(16) unsigned char tile_smem_raw[];
+    raw *sm = reinterpret_cast<raw *>(tile_smem_raw);
+    const int4 tk = B.tasks[blockIdx.x];
+    if (tk.x < 0 || tk.x >= B.n_inst) return;
+    const BatchInstanceDev in = B.inst[tk.x];
+    const long long need = 9ll * in.nx * in.ny;
+    if (in.nx <= 0 || in.ny <= 0 || in.offset < 0 || in.offset + need > B.total) return;
+    Tile<DT> t;
+    t.src = static_cast<const raw *>(B.src) + in.offset;
+    t.dst = static_cast<raw *>(B.dst) + in.offset;
+    t.nx = in.nx;
+    t.ny = in.ny;
+    t.x0 = tk.y;
+    t.y0 = tk.z;
+    t.ro = tk.w & 0xffff;
+    t.co = tk.w >> 16;
+    t.steps = B.steps;
+    t.omega = (typename Codec<DT>::real)in.omega;
+    t.u0 = (typename Codec<DT>::real)in.u0;
+    t.split_lid = false;
+    const bool whole = t.co == t.ny;
+    if (t.steps > t.nx || t.steps > t.ny || t.ro < 1 || t.co < 1 || t.x0 < 0 || t.x0 + t.ro > t.nx || t.y0 < 0 ||
+        t.y0 + t.co > t.ny || (t.ro + 2 * t.steps) * (whole ? t.ny : t.co + 2 * t.steps) > tile_plane<DT>() ||
+        (BC != LBGB_PERIODIC && (t.nx < 2 || t.ny < 2)))
+        return;
+    if (whole)
+        tile_run<DT, BC, false, true>(t, sm, nullptr, 0u, 0u);
+    else
+        tile_run<DT, BC, false, false>(t, sm, nullptr, 0u, 0u);
+}
+
+template <int DT, int BC>
+static int launch_tile_batch_v(const BatchCall &c, cudaStream_t s) {
+    static std::atomic<bool> attr_set[MAX_DEVICES];
+    const int dev = current_device();
+    if (!attr_set[dev].load(std::memory_order_acquire)) {
+        std::lock_guard<std::mutex> lock(setup_mutex());
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_tile_batch<DT, BC>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM);
+        if (e != cudaSuccess) {
+            set_error("k_tile_batch: cannot reserve %d bytes of shared memory: %s", TILE_SMEM, cudaGetErrorString(e));
+            return LBGB_ECUDA;
+        }
+        attr_set[dev].store(true, std::memory_order_release);
+    }
+    k_tile_batch<DT, BC><<<(unsigned)c.n_tasks, TILE_THREADS, TILE_SMEM, s>>>(c);
+    return check_launch("k_tile_batch");
+}
+
+template <int DT>
+int launch_tile_batch(const BatchCall &c, cudaStream_t s) {
+    switch (c.boundary) {
+    case LBGB_CAVITY: return launch_tile_batch_v<DT, LBGB_CAVITY>(c, s);
+    case LBGB_CAVITY_LADD: return launch_tile_batch_v<DT, LBGB_CAVITY_LADD>(c, s);
+    default: return launch_tile_batch_v<DT, LBGB_PERIODIC>(c, s);
     }
 }
 
