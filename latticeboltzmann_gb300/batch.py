@@ -19,7 +19,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .solver import _RAW, viscosity_from_omega
+from .solver import _RAW, capture_steps, viscosity_from_omega
 
 INSTANCE_DTYPE = np.dtype([("offset", "<i8"), ("nx", "<i4"), ("ny", "<i4"), ("omega", "<f8"), ("u0", "<f8"),
                            ("vec", "<i4"), ("cell_base", "<u4")])
@@ -309,45 +309,14 @@ class BatchedLattice:
             raise ValueError("capture: n must be a positive even number")
         self.task_queue(self.config["vector"], self.config["rows"], self.config.get("flat", False))  # outside the capture
         self._table(self.config["vector"])
-        # an odd number of launches would leave the state in the other buffer:
-        # one of them is then split in two
-        _, most = self._several()
-        plans = [(n,)]
-        for t in (-(-n // -(-n // most)), n % most or most, 2):
-            if 2 <= t <= n:
-                plans.append((n - t, t // 2, t - t // 2))
         saved = self.state.clone()
         cur, taken = self._cur, self.steps_taken
-        # the first split whose launches return to this buffer, run once outside
-        # the capture (kernels loaded, task lists on the device)
-        for parts in plans:
-            for p in parts:
-                self.step(p)
-            back = self._cur == cur
-            self._buf[cur].copy_(saved)
-            self._cur, self.steps_taken = cur, taken
-            if back:
-                break
-        else:
-            raise RuntimeError("capture: no even number of launches for %d steps" % n)
-        torch.cuda.synchronize(self.device)
-        s = torch.cuda.Stream(device=self.device)
-        s.wait_stream(torch.cuda.current_stream(self.device))
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s):
-            with torch.cuda.graph(g, stream=s):
-                for p in parts:
-                    self.step(p)
+        # run once outside the capture (kernels loaded, task lists on the device)
+        self.step(n)
+        self._buf[cur].copy_(saved)
         self._cur, self.steps_taken = cur, taken
-        torch.cuda.current_stream(self.device).wait_stream(s)
-        batch = self
-
-        def replay():
-            g.replay()
-            batch.steps_taken += n
-
-        replay.graph = g
-        return replay
+        torch.cuda.synchronize(self.device)
+        return capture_steps(self, n)
 
     # ------------------------------------------------------------ diagnostics
     def shear_amplitudes(self, out=None):

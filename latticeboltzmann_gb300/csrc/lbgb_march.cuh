@@ -235,29 +235,39 @@ struct March {
     uint4 *in, *delay;  // this lane's vector of [channel] and [step][plane], 32 lanes each
     f32x2 omega;
     float u0;
-    int col[MODE == MARCH_VECTORS ? 1 : 4];  // RAG: columns of cells 32 i + lane of the warp's 128; GRP: of the lane's cells
+    int col[MODE == MARCH_VECTORS ? 1 : 4];  // columns of cells 32 i + lane of the warp's 128
+    int row0[GRP ? 4 : 1];                    // GRP: rows of their group beyond this lane's
     uint32_t key[T];
 
     __device__ __forceinline__ int wrap(int r) const { return r < 0 ? r + nx : (r >= nx ? r - nx : r); }
 
     // copies the pulled rows of lattice row r (channel i from row r - cx_i)
     __device__ __forceinline__ void issue(int r) const {
-        const int c = RAG || (GRP && !K.vec) ? 0 : K.c;
-        const raw *q0 = src + (size_t)wrap(r) * ny + c, *qm = src + (size_t)wrap(r - 1) * ny + c,
-                  *qp = src + (size_t)wrap(r + 1) * ny + c;
+        if (MODE == MARCH_VECTORS || (GRP && K.vec)) {
+            const raw *q0 = src + (size_t)wrap(r) * ny + K.c, *qm = src + (size_t)wrap(r - 1) * ny + K.c,
+                      *qp = src + (size_t)wrap(r + 1) * ny + K.c;
 #pragma unroll
-        for (int ch = 0; ch < 9; ++ch) {
-            const raw *q = (cx(ch) == 0 ? q0 : (cx(ch) > 0 ? qm : qp)) + ch * cs;
-            if constexpr (RAG) {
-                float *s = reinterpret_cast<float *>(in - lane + ch * 32) + lane;
+            for (int ch = 0; ch < 9; ++ch)
+                cp_async16(in + ch * 32, (cx(ch) == 0 ? q0 : (cx(ch) > 0 ? qm : qp)) + ch * cs);
+            return;
+        }
+        // element by element, 32 neighbours at a time: cell 32 i + lane of the
+        // warp's 128 (each lane its own four cells took four times the
+        // wavefronts); GRP: of the group that these cells belong to
+        if constexpr (MODE != MARCH_VECTORS) {
+            float *s = reinterpret_cast<float *>(in - lane) + lane;
+            const raw *q0, *qm, *qp;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) cp_async4(s + 32 * i, q + col[i]);
-            } else if (GRP && !K.vec) {
-                float *s = reinterpret_cast<float *>(in + ch * 32);
+            for (int i = 0; i < 4; ++i) {
+                if (i == 0 || (GRP && K.width < 32)) {
+                    const int k = GRP ? r + row0[GRP ? i : 0] : r;
+                    q0 = src + (size_t)wrap(k) * ny;
+                    qm = src + (size_t)wrap(k - 1) * ny;
+                    qp = src + (size_t)wrap(k + 1) * ny;
+                }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) cp_async4(s + i, q + col[GRP ? i : 0]);
-            } else {
-                cp_async16(in + ch * 32, q);
+                for (int ch = 0; ch < 9; ++ch)
+                    cp_async4(s + ch * 128 + 32 * i, (cx(ch) == 0 ? q0 : (cx(ch) > 0 ? qm : qp)) + ch * cs + col[i]);
             }
         }
     }
@@ -292,7 +302,7 @@ struct March {
         {
             uint32_t v[9][4];
             cp_async_wait<0>();
-            if (RAG) __syncwarp();
+            if (MODE != MARCH_VECTORS) __syncwarp();
 #pragma unroll
             for (int ch = 0; ch < 9; ++ch) ld_words(in + ch * 32, v[ch]);
 #pragma unroll
@@ -318,7 +328,7 @@ struct March {
             }
             march_collide<DT, SRND, EDGE>(v, omega, lid, jt, key[0], (uint32_t)((size_t)k * ny + K.c), o);
             // the row's values are in registers: the next row takes its place
-            if (RAG) __syncwarp();
+            if (MODE != MARCH_VECTORS) __syncwarp();
             if (it + 1 < iters) issue(r_first + it + 1);
             cp_async_commit();
         }
@@ -571,8 +581,13 @@ __global__ void __launch_bounds__(MARCH_WPB * 32, MARCH_WARPS / MARCH_WPB) k_mar
     const bool edge = WALLS && __any_sync(0xffffffffu, K.bottom || K.top);
     K.c %= in.ny;
     if (K.c < 0) K.c += in.ny;
+    // cells 32 i + lane of the warp's 128: first column and row of their group
 #pragma unroll
-    for (int i = 0; i < 4; ++i) M.col[i] = (K.c + i) % in.ny;
+    for (int i = 0; i < 4; ++i) {
+        const int e = 32 * i + lane, first = (e / (4 * width)) * width;
+        M.col[i] = (__shfl_sync(0xffffffffu, K.c, first) + e % (4 * width)) % in.ny;
+        M.row0[i] = __shfl_sync(0xffffffffu, K.X0, first) - K.X0;
+    }
     M.K = K;
     M.r_first = K.X0 - (T - 1);
     M.iters = rows + 2 * (T - 1);

@@ -38,6 +38,40 @@ def viscosity_from_omega(omega):
     return (1.0 / omega - 0.5) / 3.0
 
 
+def capture_steps(lattice, n):
+    """CUDA graph of ``lattice.step(n)``; returns a callable replaying it.
+
+    A graph holds the addresses of the two buffers.  Where the launches of n
+    steps (several steps each) are odd in number, the state ends in the other
+    buffer: a second graph starts from there, and the replays alternate."""
+    graphs = {}
+    start = lattice._cur
+    for cur in (start, 1 - start):
+        lattice._cur = cur
+        s = torch.cuda.Stream(device=lattice.device)
+        s.wait_stream(torch.cuda.current_stream(lattice.device))
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(s):
+            with torch.cuda.graph(g, stream=s):
+                lattice.step(n)
+        torch.cuda.current_stream(lattice.device).wait_stream(s)
+        lattice.steps_taken -= n
+        graphs[cur] = (g, lattice._cur)
+        if lattice._cur == cur:
+            break
+    lattice._cur = start
+
+    def replay():
+        g, end = graphs.get(lattice._cur) or graphs[start]
+        g.replay()
+        if len(graphs) == 2:
+            lattice._cur = end
+        lattice.steps_taken += n
+
+    replay.graph = graphs[start][0]
+    return replay
+
+
 class Lattice:
     """A ``(9, nx, ny)`` D2Q9 lattice resident on one GPU.
 
@@ -119,9 +153,6 @@ class Lattice:
         if self.rounding == "stochastic" and self.storage in ("f16dev", "bf16dev"):
             return 1
         return int(_lib.load().lbgb_steps_per_launch(self.nx, self.ny, self.bcode, self.code))
-
-    def _max_steps_per_launch(self):
-        return int(_lib.load().lbgb_max_steps_per_launch(self.nx, self.ny, self.bcode, self.code))
 
     @property
     def state(self):
@@ -339,8 +370,7 @@ class Lattice:
     def capture(self, n):
         """Capture ``n`` steps into a CUDA graph; returns a callable replaying them.
 
-        ``n`` must be even so that the state returns to the same buffer after
-        each replay (the graph bakes the buffer addresses in).
+        ``n`` must be even.
         """
         if n <= 0 or n % 2:
             raise ValueError("capture: n must be a positive even number")
@@ -355,35 +385,7 @@ class Lattice:
                       self.omega, self.u0, self.code, 1, self.seed, ctr.data_ptr(), ctypes.byref(ctypes.c_int(0)),
                       self._stream())
         torch.cuda.current_stream(self.device).synchronize()
-        cur = self._cur
-        # an odd number of launches of several steps each would leave the
-        # state in the other buffer: one of them is then split in two
-        most = self._max_steps_per_launch()
-        plans = [(n,)]
-        for t in (-(-n // -(-n // most)), n % most or most, 2):
-            if 2 <= t <= n:
-                plans.append((n - t, t // 2, t - t // 2))
-        for parts in plans + [(1,) * n]:
-            s = torch.cuda.Stream(device=self.device)
-            s.wait_stream(torch.cuda.current_stream(self.device))
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.stream(s):
-                with torch.cuda.graph(g, stream=s):
-                    for p in parts:
-                        self.step(p)
-            self.steps_taken -= n
-            if self._cur == cur:
-                break
-            self._cur = cur
-        torch.cuda.current_stream(self.device).wait_stream(s)
-        lattice = self
-
-        def replay():
-            g.replay()
-            lattice.steps_taken += n
-
-        replay.graph = g
-        return replay
+        return capture_steps(self, n)
 
     # ------------------------------------------------------------------ diagnostics
     def macroscopic(self):
