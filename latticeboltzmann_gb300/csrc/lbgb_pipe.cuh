@@ -6,13 +6,15 @@
 // warps 0..NCW-1 (the consumers) gather every population of their cells from
 // the stage, release it, collide and store straight to global memory.
 //
-// A tile is L = NCW*32*NC consecutive cells of one row k (NC = cells per
-// consumer thread = one 16-byte vector).  For channel i the producer copies
-// row k - cx_i (or, at a cavity side wall, the opposite channel of row k),
-// columns [l0 - HALO, l0 + L + HALO) clipped to the row, HALO = one 16-byte
-// vector: the one-cell neighbours along l that the cy != 0 channels pull are
-// then in shared memory.  Only the cells of the first and last column of a
-// row fetch their wrap-around or wall values from global memory.
+// A tile is NCW segments of 32*NC consecutive cells of a row (NC = cells per
+// consumer thread = one 16-byte vector), one per consumer warp: segments of
+// one row k, or (SPAN) NCW consecutive segments of the lattice, whatever rows
+// they are in.  For channel i the producer copies row k - cx_i (or, at a
+// cavity side wall, the opposite channel of row k), the run of cells
+// [l0 - HALO, l1 + HALO) clipped to the row, HALO = one 16-byte vector: the
+// one-cell neighbours along l that the cy != 0 channels pull are then in
+// shared memory.  Only the cells of the first and last column of a row fetch
+// their wrap-around or wall values from global memory.
 //
 // A stage holds ~37 KB (FP32: 9 channels x 1032 cells); with the default
 // two stages ~74 KB per SM are in flight, independent of how long the
@@ -37,8 +39,8 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
+__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
@@ -65,6 +67,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
 __device__ __forceinline__ void prefetch_l1(const void *p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
+                 : "memory");
+}
 // Bulk asynchronous copy global -> shared, completion counted on `bar`.
 __device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -81,42 +87,57 @@ constexpr long long PIPE_DRAIN_LIMIT = 1ll << 22;
 __device__ __forceinline__ void pipe_report(int code) { atomicCAS(&g_pipe_status, 0, code); }
 
 // Tile geometry: NCW consumer warps, NC cells per consumer thread (one 8- or
-// 16-byte packet per channel), a 16-byte halo on each side of the row segment
-// (bulk copies start and end on 16-byte boundaries).
-template <class RAW, int NCW_, int NC_>
+// 16-byte packet per channel), a 16-byte halo on each side of a run of cells
+// (bulk copies start and end on 16-byte boundaries).  A tile that spans rows
+// has at most one run per segment.
+template <class RAW, int NCW_, int NC_, bool SPAN>
 struct PipeGeom {
     static constexpr int NCW = NCW_;
     static constexpr int NC = NC_;
     static constexpr int HALO = 16 / (int)sizeof(RAW);
-    static constexpr int L = NCW * 32 * NC;                    // cells per tile
-    static constexpr int SLOT = L + 2 * HALO;                  // elements per channel slot
+    static constexpr int SEG = 32 * NC;                        // cells per segment
+    static constexpr int SLOT = NCW * SEG + 2 * HALO * (SPAN ? NCW : 1);  // elements per channel slot
     static constexpr size_t STAGE_BYTES = 9ull * SLOT * sizeof(RAW);
 };
 
-// Shapes per storage code: FP32 8 warps x 4 cells, FP64 8 x 2; the 16-bit
-// codecs have twice the cells per byte, so 8 warps hold 8 cells each (more
-// work per thread between the per-tile fixed costs; 168 registers, no
-// spills).  CTAS: resident CTAs per SM (the launch bound and the persistent
-// grid).  Measured at 8192^2 (FP16, FP16 stochastic, BF16 MLUPS): 8 x 8 with
-// one CTA 163.8k / 154.7k / 168.4k; 8 x 4 with two CTAs (96 registers)
-// 153.4k / 136.8k / 151.8k; 16 x 4 with one CTA 158.4k / 146.6k / 160.6k.
-template <int DT> struct PipeShape { static constexpr int NCW = 8, NC = 4, CTAS = 1; };
-template <> struct PipeShape<LBGB_F64> { static constexpr int NCW = 8, NC = 2, CTAS = 1; };
-template <> struct PipeShape<LBGB_F16DEV> { static constexpr int NCW = 8, NC = 8, CTAS = 1; };
-template <> struct PipeShape<LBGB_BF16DEV> { static constexpr int NCW = 8, NC = 8, CTAS = 1; };
+// Shapes per storage code: FP32 8 warps x 4 cells; the 16-bit codecs have
+// twice the cells per byte, so 8 warps hold 8 cells each (more work per thread
+// between the per-tile fixed costs; 168 registers, no spills).  CTAS: resident
+// CTAs per SM (the launch bound and the persistent grid).  Measured at 8192^2
+// (FP16, FP16 stochastic, BF16 MLUPS): 8 x 8 with one CTA 163.8k / 154.7k /
+// 168.4k; 8 x 4 with two CTAs (96 registers) 153.4k / 136.8k / 151.8k; 16 x 4
+// with one CTA 158.4k / 146.6k / 160.6k.
+//
+// FP64: the fixed-point collision is a long chain of integer and FP64
+// operations (ALU 43 %, FP64 pipe 46 % with 8 warps), so the SM wants warps:
+// 15 x 2 cells, all that fit with 128 registers a thread.  Tiles of 960 cells
+// fit few rows (3 of them for 2048 cells: 71 % of the lanes work), so they span
+// rows.  us a step at 1024^2, 2048^2, 3000^2, 4096^2, 8192^2: 8 warps 57.5, 198,
+// 346, 770, -; 15 warps within a row 63.8, 158, 318, 513, 1842; 15 warps
+// spanning 43.1, 129, 256, 468, 1818; 12 warps spanning 44.2, 152, 275, 534,
+// 2023; two CTAs of 7 spanning 46.5, 144, 285, 531, 2078; every warp a
+// pipeline of its own, no producer: 43.8, 156, 286, 601, 2381 (its copies are
+// 544 bytes).  16-bit tiles that span rows measured 0-2 % slower at 4096^2,
+// whose rows are whole tiles, and 14-24 % faster at 8192x1000; several steps of
+// those are k_march's, so theirs stay within a row.
+template <int DT> struct PipeShape { static constexpr int NCW = 8, NC = 4, CTAS = 1; static constexpr bool SPAN = false; };
+template <> struct PipeShape<LBGB_F64> { static constexpr int NCW = 15, NC = 2, CTAS = 1; static constexpr bool SPAN = true; };
+template <> struct PipeShape<LBGB_F16DEV> { static constexpr int NCW = 8, NC = 8, CTAS = 1; static constexpr bool SPAN = false; };
+template <> struct PipeShape<LBGB_BF16DEV> { static constexpr int NCW = 8, NC = 8, CTAS = 1; static constexpr bool SPAN = false; };
 
 template <int DT, int BC, bool COLLIDE, int NCW_, int NC_, bool SRND>
 __global__ void __launch_bounds__((NCW_ + 1) * 32, PipeShape<DT>::CTAS)
 k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>::raw *__restrict__ dst, int nx,
-            int ny, int tiles_per_row, int total_tiles, int stages, typename Codec<DT>::real omega,
+            int ny, int row_segs, int total_segs, int stages, typename Codec<DT>::real omega,
             typename Codec<DT>::real u0, long long wait_limit, int stall_producer,
             const unsigned long long *__restrict__ sr_step, uint32_t sr_seed, uint32_t sr_offset, int k_first) {
     using C = Codec<DT>;
     using raw = typename C::raw;
     using real = typename C::real;
-    using G = PipeGeom<raw, NCW_, NC_>;
+    constexpr bool SPAN = PipeShape<DT>::SPAN;
+    using G = PipeGeom<raw, NCW_, NC_, SPAN>;
     using P = Packet<DT, NC_>;
-    constexpr int NC = G::NC, HALO = G::HALO, L = G::L, SLOT = G::SLOT, NCW = G::NCW;
+    constexpr int NC = G::NC, HALO = G::HALO, SEG = G::SEG, SLOT = G::SLOT, NCW = G::NCW;
     // FP16 collisions run in the stored units (deviations times 2^14): no
     // scaling per value on decode or encode, bit for bit the same results
     constexpr bool UNITS = DT == LBGB_F16DEV && COLLIDE;
@@ -135,6 +156,19 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t cs = (size_t)nx * ny;
+    // first segment of the block's tile: row fr, segment fs of the row, advanced
+    // without a division per tile
+    const int total_tiles = (total_segs + NCW - 1) / NCW, step = gridDim.x * NCW;
+    const int dq = step / row_segs, dr = step - dq * row_segs;
+    int fr = blockIdx.x * NCW / row_segs, fs = blockIdx.x * NCW - fr * row_segs;
+    auto advance = [&]() {
+        fr += dq;
+        fs += dr;
+        if (fs >= row_segs) {
+            fs -= row_segs;
+            ++fr;
+        }
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -159,24 +193,35 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
                 pipe_report(1);
                 break;
             }
-            const int k = k_first + tile / tiles_per_row;
-            const int l0 = (tile - (k - k_first) * tiles_per_row) * L;
-            const int c0 = max(l0 - HALO, 0), c1 = min(l0 + L + HALO, ny);
-            const uint32_t bytes = (uint32_t)(c1 - c0) * (uint32_t)sizeof(raw);
-            mbar_arrive_expect_tx(&full[s], 9u * bytes);
             raw *stage = slots + (size_t)s * 9 * SLOT;
+            int k = k_first + fr, sg = fs;
+            // one run of segments per row that the tile reaches
+            for (int left = min(NCW, total_segs - tile * NCW); left > 0; ++k, sg = 0) {
+                const int n = SPAN ? min(left, row_segs - sg) : NCW;
+                const int l0 = sg * SEG;
+                const int c0 = max(l0 - HALO, 0), c1 = min(l0 + n * SEG + HALO, ny);
+                const uint32_t bytes = (uint32_t)(c1 - c0) * (uint32_t)sizeof(raw);
+                if constexpr (SPAN)
+                    mbar_expect_tx(&full[s], 9u * bytes);
+                else
+                    mbar_arrive_expect_tx(&full[s], 9u * bytes);
 #pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                int ch = i, row = k - cx(i);
-                if (BC == LBGB_PERIODIC) {
-                    row = row < 0 ? row + nx : (row >= nx ? row - nx : row);
-                } else if (row < 0 || row >= nx) {
-                    ch = opp(i);
-                    row = k;
+                for (int i = 0; i < 9; ++i) {
+                    int ch = i, row = k - cx(i);
+                    if (BC == LBGB_PERIODIC) {
+                        row = row < 0 ? row + nx : (row >= nx ? row - nx : row);
+                    } else if (row < 0 || row >= nx) {
+                        ch = opp(i);
+                        row = k;
+                    }
+                    bulk_copy_g2s(stage + i * SLOT + (c0 - (l0 - HALO)), src + (size_t)ch * cs + (size_t)row * ny + c0,
+                                  bytes, &full[s]);
                 }
-                bulk_copy_g2s(stage + i * SLOT + (c0 - (l0 - HALO)), src + (size_t)ch * cs + (size_t)row * ny + c0,
-                              bytes, &full[s]);
+                left -= n;
+                stage += n * SEG + 2 * HALO;
             }
+            if constexpr (SPAN) mbar_arrive(&full[s]);
+            advance();
             ++issued;
         }
         // drain: the copies of the last stages issued must land before exit
@@ -186,21 +231,23 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
     }
 
     // ---------------------------------------------------------------- consumers
-    const int t = threadIdx.x;  // 0 .. NCW*32-1
-    // tile -> (row, tile within the row), advanced without a division per tile
-    const int dq = gridDim.x / tiles_per_row, dr = gridDim.x - dq * tiles_per_row;
-    int kr = blockIdx.x / tiles_per_row, lt = blockIdx.x - kr * tiles_per_row;
+    // this warp's segment of the tile: row k, first cell l0, rows reached before it
+    int k_next, l0_next, run_next;
+    auto locate = [&]() {
+        const int sg = fs + warp;
+        run_next = SPAN && sg >= row_segs ? sg / row_segs : 0;
+        k_next = k_first + fr + run_next;
+        l0_next = (sg - run_next * row_segs) * SEG;
+    };
     // The threads at a row's first and last column read a few values from
     // global memory after the stage wait (wrap-around, walls, the lid
     // density).  Their addresses are prefetched into L1 one tile ahead, so
     // that those warps do not wait a DRAM round trip while holding a stage.
     // (16-bit storage: not done -- those kernels are issue-bound, and the
     // per-tile instructions cost more than the stalls they save: -4 %)
-    auto prefetch_edges = [&](int tl, int krow, int ltile) {
+    auto prefetch_edges = [&](int tl, int kk, int cc) {
         if constexpr (sizeof(raw) == 2) return;
-        if (tl >= total_tiles) return;
-        const int kk = k_first + krow;
-        const int cc = ltile * L + t * NC;
+        if (tl * NCW + warp >= total_segs) return;
         const bool first = cc == 0, last = cc + NC == ny;
         if (!first && !last) return;
         auto pf = [&](int ch, int row, int l) { prefetch_l1(src + (size_t)ch * cs + (size_t)row * ny + l); };
@@ -239,34 +286,31 @@ k_step_pipe(const typename Codec<DT>::raw *__restrict__ src, typename Codec<DT>:
             }
         }
     };
-    prefetch_edges(blockIdx.x, kr, lt);
+    locate();
+    prefetch_edges(blockIdx.x, k_next, l0_next + lane * NC);
     int it = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
-        const int k = k_first + kr;
-        const int l0 = lt * L;
-        lt += dr;
-        kr += dq;
-        if (lt >= tiles_per_row) {
-            lt -= tiles_per_row;
-            ++kr;
-        }
-        prefetch_edges(tile + gridDim.x, kr, lt);
+        const int k = k_next, l0 = l0_next, run = run_next;
+        advance();
+        locate();
+        prefetch_edges(tile + gridDim.x, k_next, l0_next + lane * NC);
+        const bool mine = !SPAN || tile * NCW + warp < total_segs;
         const int s = it % stages;
         const uint32_t ph = (uint32_t)(it / stages) & 1u;
         if (!mbar_wait(&full[s], ph, wait_limit)) {
             pipe_report(2);
             break;
         }
-        const int c = l0 + t * NC;  // first cell of this thread
-        const bool act = c < ny;
-        const raw *stage = slots + (size_t)s * 9 * SLOT;
+        const int c = l0 + lane * NC;  // first cell of this thread
+        const bool act = mine && c < ny;
+        const raw *stage = slots + (size_t)s * 9 * SLOT + warp * SEG + run * 2 * HALO;
         const bool wl = (BC != LBGB_PERIODIC) && k == 0;
         const bool wr = (BC != LBGB_PERIODIC) && k == nx - 1;
         real v[9][NC];
         if (act) {
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
-                const raw *sl = stage + i * SLOT + HALO + t * NC;
+                const raw *sl = stage + i * SLOT + HALO + lane * NC;
                 if constexpr (UNITS)
                     P::dec_units(*reinterpret_cast<const typename P::vec *>(sl), v[i]);
                 else

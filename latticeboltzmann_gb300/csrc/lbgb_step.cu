@@ -390,17 +390,19 @@ static int launch_pipe(const void *src, void *dst, int nx, int ny, double omega,
                        SR sr, Rows rows) {
     using raw = typename Codec<DT>::raw;
     using SH = PipeShape<DT>;
-    using G = PipeGeom<raw, SH::NCW, SH::NC>;
-    const long long tpr = (ny + G::L - 1) / G::L;
-    const long long total = (long long)rows.n(nx) * tpr;
+    using G = PipeGeom<raw, SH::NCW, SH::NC, SH::SPAN>;
+    long long row_segs = (ny + G::SEG - 1) / G::SEG;
+    if (!SH::SPAN) row_segs = (row_segs + SH::NCW - 1) / SH::NCW * SH::NCW;  // whole tiles
+    const long long segs = (long long)rows.n(nx) * row_segs;
     const int smax = max_dyn_smem();
     const int fit = (int)((smax / SH::CTAS - 256) / (G::STAGE_BYTES + 16));
     int stages = (int)g_tune.stages;
     if (stages > fit) stages = fit;
-    if (stages < 2 || total > INT_MAX) return 1;  // caller falls back to the register kernel
+    if (stages < 2 || segs > INT_MAX / 2) return 1;  // caller falls back to the register kernel
     const size_t smem = (size_t)stages * G::STAGE_BYTES + 16 * (size_t)stages;
     const long long slots = (long long)sm_count() * SH::CTAS;
-    const int grid = (int)(total < slots ? total : slots);
+    const long long tiles = (segs + SH::NCW - 1) / SH::NCW;
+    const int grid = (int)(tiles < slots ? tiles : slots);
     const bool srnd = sizeof(raw) == 2 && COLLIDE && sr.step != nullptr;
     // the dynamic shared-memory limit is raised once per kernel variant and device
     static std::atomic<bool> attr_set[MAX_DEVICES][2];
@@ -416,7 +418,7 @@ static int launch_pipe(const void *src, void *dst, int nx, int ny, double omega,
             attr_set[dev][variant].store(true, std::memory_order_release);
         }
         kernel<<<grid, (SH::NCW + 1) * 32, smem, s>>>(
-            static_cast<const raw *>(src), static_cast<raw *>(dst), nx, ny, (int)tpr, (int)total, stages,
+            static_cast<const raw *>(src), static_cast<raw *>(dst), nx, ny, (int)row_segs, (int)segs, stages,
             (typename Codec<DT>::real)omega, (typename Codec<DT>::real)u0, g_tune.wait_limit,
             (int)g_tune.stall_producer, sr.step, sr.seed, sr.offset, rows.first);
         return LBGB_OK;
