@@ -431,6 +431,34 @@ LBGB_API int lbgb_fno_mix(const float *P, const void *Rr, const void *Ri, void *
                           int q, int mk, void *stream);
 LBGB_API int lbgb_fno_mix_back(const float *dYm, const float *P, const void *Rr, const void *Ri, void *dP,
                                float *dRr, float *dRi, int C, int O, int B, int q, int mk, void *stream);
+/* The surrogate's layers with what follows them, on channel-major BF16
+ * activations (channels, rows * w), w a multiple of 8, 16-byte aligned:
+ *   D(p, n) = sum_j a2(j, p % w) b2(n, p / w, j) + sum_k x(k, p) b1[n * b1_ns + k * b1_ks]
+ * (x (k1, rows * w), a2 (k2, w), b2 (n, rows, k2), k1 <= 128, k2 <= 64 and a
+ * multiple of 8; k2 = 0 leaves the first sum out), two FP32 sums.
+ *   layer         z = D + bias (FP32, null: not stored), v = BF16(act ? gelu(z) : z); n <= 32
+ *   layer_back    dz = BF16(z ? D gelu'(z) : D), sums[n] = its sum over the pixels before the
+ *                 rounding; n <= 32
+ *   project       h = x q1 + q1b, g = BF16(gelu(h)) (null: not stored), out (cout <= 4, rows * w) =
+ *                 q2 g + q2b (null: not computed); n <= 128 hidden channels
+ *   project_back  dh = BF16((q2^T d) gelu'(h)), d BF16 (cout <= 64, rows * w), with h computed
+ *                 again; sums as above
+ * The sums are lbgb_fno_row_sum's, addition for addition; f32 (n, rows * w), 16-byte
+ * aligned, receives the values summed, and may be null where lbgb_fno_layer_sums is 1
+ * (k2 = 0 for project_back).  n is a multiple of 16, z 16-byte aligned.  parts: lbgb_fno_layer_parts(n) floats of scratch. */
+LBGB_API int lbgb_fno_layer(int n, int k1, int rows, int w, const void *x, const void *b1, long long b1_ns,
+                            long long b1_ks, int k2, const void *a2, const void *b2, const float *bias, int act,
+                            float *z, void *v, void *stream);
+LBGB_API int lbgb_fno_layer_back(int n, int k1, int rows, int w, const void *x, const void *b1, long long b1_ns,
+                                 long long b1_ks, int k2, const void *a2, const void *b2, const float *z, void *dz,
+                                 float *f32, float *sums, float *parts, void *stream);
+LBGB_API int lbgb_fno_project(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
+                              int cout, const void *q2, const float *q2b, void *g, float *out, void *stream);
+LBGB_API int lbgb_fno_project_back(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
+                                   int cout, const void *q2, const void *d, void *dh, float *f32, float *sums,
+                                   float *parts, void *stream);
+LBGB_API long long lbgb_fno_layer_parts(int n);
+LBGB_API int lbgb_fno_layer_sums(int rows, int w, int k2);
 LBGB_API int lbgb_fno_mse(const float *y, const float *t, float *d, double *partials, int nparts,
                           long long n, void *stream);
 /* lbgb_fno_mse with a weight per plane of `plane` consecutive elements (the

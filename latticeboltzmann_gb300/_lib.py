@@ -89,6 +89,14 @@ SIGNATURES = {
     "lbgb_fno_row_sum": (_I, [_P, _P, _P, _I, ctypes.c_longlong, _P]),
     "lbgb_fno_mix": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),
     "lbgb_fno_mix_back": (_I, [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P]),
+    "lbgb_fno_layer": (_I, [_I, _I, _I, _I, _P, _P, ctypes.c_longlong, ctypes.c_longlong, _I, _P, _P, _P, _I, _P, _P,
+                            _P]),
+    "lbgb_fno_layer_back": (_I, [_I, _I, _I, _I, _P, _P, ctypes.c_longlong, ctypes.c_longlong, _I, _P, _P, _P, _P, _P,
+                                 _P, _P, _P]),
+    "lbgb_fno_project": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _P]),
+    "lbgb_fno_project_back": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P]),
+    "lbgb_fno_layer_parts": (ctypes.c_longlong, [_I]),
+    "lbgb_fno_layer_sums": (_I, [_I, _I, _I]),
     "lbgb_fno_mse": (_I, [_P, _P, _P, _P, _I, ctypes.c_longlong, _P]),
     "lbgb_fno_mse_weighted": (_I, [_P, _P, _P, ctypes.c_longlong, _P, _P, _I, ctypes.c_longlong, _P]),
     "lbgb_fno_adam": (_I, [_P, _P, _P, _P, _P, ctypes.c_longlong, ctypes.c_float, ctypes.c_float, ctypes.c_float,

@@ -985,6 +985,8 @@ static int launch_gemm(int m, int n, int k, const __nv_bfloat16 *a, long long a_
 
 }  // namespace lbgb
 
+#include "lbgb_layer.cuh"
+
 using namespace lbgb;
 
 extern "C" int lbgb_gemm_bf16(int m, int n, int k, const void *A, long long a_rs, long long a_cs, long long a_bs,
@@ -1041,6 +1043,68 @@ extern "C" int lbgb_gemm_bf16_bias_act(int m, int n, int k, const void *A, long 
     }
     return rc;
 }
+
+extern "C" int lbgb_fno_layer(int n, int k1, int rows, int w, const void *x, const void *b1, long long b1_ns,
+                              long long b1_ks, int k2, const void *a2, const void *b2, const float *bias, int act,
+                              float *z, void *v, void *stream) {
+    if (!x || !b1 || !v || (k2 > 0 && (!a2 || !b2)) || !aligned(v, 4)) {
+        set_error("lbgb_fno_layer: null or misaligned operand");
+        return LBGB_EINVAL;
+    }
+    LayerArgs a{};
+    a.n = n, a.k1 = k1, a.k2 = k2, a.rows = rows, a.W = w;
+    a.b1 = static_cast<const __nv_bfloat16 *>(b1), a.b1_ns = b1_ns, a.b1_ks = b1_ks;
+    a.bias = bias, a.act = act, a.z = z, a.v = static_cast<__nv_bfloat16 *>(v);
+    return launch_layer<LAYER>(a, x, a2, b2, nullptr, (cudaStream_t)stream, "lbgb_fno_layer");
+}
+
+extern "C" int lbgb_fno_layer_back(int n, int k1, int rows, int w, const void *x, const void *b1, long long b1_ns,
+                                   long long b1_ks, int k2, const void *a2, const void *b2, const float *z, void *dz,
+                                   float *f32, float *sums, float *parts, void *stream) {
+    if (!x || !b1 || !dz || !sums || !parts || (k2 > 0 && (!a2 || !b2)) || !aligned(dz, 4)) {
+        set_error("lbgb_fno_layer_back: null or misaligned operand");
+        return LBGB_EINVAL;
+    }
+    LayerArgs a{};
+    a.n = n, a.k1 = k1, a.k2 = k2, a.rows = rows, a.W = w;
+    a.b1 = static_cast<const __nv_bfloat16 *>(b1), a.b1_ns = b1_ns, a.b1_ks = b1_ks;
+    a.z = const_cast<float *>(z), a.v = static_cast<__nv_bfloat16 *>(dz);
+    a.f32 = f32, a.parts = parts;
+    return launch_layer<BACK>(a, x, a2, b2, sums, (cudaStream_t)stream, "lbgb_fno_layer_back");
+}
+
+extern "C" int lbgb_fno_project(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
+                                int cout, const void *q2, const float *q2b, void *g, float *out, void *stream) {
+    if (!x || !q1 || !q1b || (!g && !out) || (out && (!q2 || !q2b)) || (g && !aligned(g, 4))) {
+        set_error("lbgb_fno_project: null or misaligned operand");
+        return LBGB_EINVAL;
+    }
+    LayerArgs a{};
+    a.n = n, a.k1 = k1, a.rows = rows, a.W = w;
+    a.b1 = static_cast<const __nv_bfloat16 *>(q1), a.b1_ns = k1, a.b1_ks = 1;
+    a.bias = q1b, a.cout = cout, a.q2 = static_cast<const __nv_bfloat16 *>(q2), a.q2b = q2b;
+    a.v = static_cast<__nv_bfloat16 *>(g), a.out = out;
+    return launch_layer<PROJECT>(a, x, nullptr, nullptr, nullptr, (cudaStream_t)stream, "lbgb_fno_project");
+}
+
+extern "C" int lbgb_fno_project_back(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
+                                     int cout, const void *q2, const void *d, void *dh, float *f32, float *sums,
+                                     float *parts, void *stream) {
+    if (!x || !q1 || !q1b || !q2 || !d || !dh || !sums || !parts || cout < 1 || !aligned(dh, 4)) {
+        set_error("lbgb_fno_project_back: null or misaligned operand");
+        return LBGB_EINVAL;
+    }
+    LayerArgs a{};
+    a.n = n, a.k1 = k1, a.rows = rows, a.W = w;
+    a.b1 = static_cast<const __nv_bfloat16 *>(q1), a.b1_ns = k1, a.b1_ks = 1;
+    a.bias = q1b, a.k2 = cout, a.q2 = static_cast<const __nv_bfloat16 *>(q2);
+    a.v = static_cast<__nv_bfloat16 *>(dh), a.f32 = f32, a.parts = parts;
+    return launch_layer<PROJECT_BACK>(a, x, d, nullptr, sums, (cudaStream_t)stream, "lbgb_fno_project_back");
+}
+
+extern "C" long long lbgb_fno_layer_parts(int n) { return n > 0 ? 256ll * SUM_CHUNKS * n : 0; }
+
+extern "C" int lbgb_fno_layer_sums(int rows, int w, int k2) { return rows > 0 && w > 0 && layer_chunk(rows, w, k2 > 0) > 0; }
 
 extern "C" int lbgb_gemm_status(int reset) {
     cudaError_t e = cudaDeviceSynchronize();

@@ -95,9 +95,8 @@ class FNO2d:
         if max_splits < 1 or max_splits & (max_splits - 1):
             raise ValueError("max_splits must be a power of two")
         self.max_splits = int(max_splits)  # weight gradients: split-K count over the pixels
-        # bias + activation in the epilogue of each layer's last GEMM (tensor-
-        # core engine; 16 x 256^2: training step 3.95 against 4.03 ms, forward
-        # 1.54 against 1.62 ms with a separate pass)
+        # layers whose products, bias, activation and its gradient are one kernel
+        # each (tensor-core engine, see _fused); False: one pass per operation
         self.fused_epilogue = True
         shapes = [("P", (width, cin)), ("pb", (width,))]
         for l in range(layers):
@@ -217,6 +216,16 @@ class FNO2d:
         self._gemm(m, n, k, A, (a[0], a[1], 0), B, (1, b_cs, 0), C, (c_rs, 1, 0), beta=1.0)
         _lib.call("lbgb_fno_bias_act", C, bias, None, None, vb, channels, cols, act, s)
 
+    def _fused(self, B, H, W):
+        """Whether every layer runs as one kernel (lbgb_fno_layer and the others):
+        the sizes those take, and rows that fill at least a quarter of their
+        128-pixel tiles (at 16 x 256^2 such a kernel takes 0.28 of the time of its
+        separate passes; 6 x 96 x 32: training 830 -> 661 us)."""
+        return (self.engine == ENGINE_TENSOR_CORES and self.fused_epilogue and W % 8 == 0
+                and 4 * W >= 128 * (-(-W // 128)) and B * H * W <= 1 << 30
+                and self.width <= 32 and self.width % 16 == 0 and 2 * self.modes <= 64 and self.modes % 4 == 0
+                and self.cin <= 128 and self.hidden <= 128 and self.hidden % 16 == 0 and self.cout <= 4)
+
     def _splits(self, K):
         """Split count of a weight gradient over K pixels: the largest power of
         two up to ``max_splits`` that divides K and leaves >= 256 per split."""
@@ -249,7 +258,8 @@ class FNO2d:
         return self._mats[key]
 
     def _workspace(self, B, H, W, train):
-        key = (B, H, W, train)
+        fused = self._fused(B, H, W)
+        key = (B, H, W, train, fused)
         if key in self._ws:
             return self._ws[key]
         # keep at most a couple of shapes alive
@@ -261,25 +271,37 @@ class FNO2d:
         bf = dict(dtype=torch.bfloat16, device=self.device)
         f32 = dict(dtype=torch.float32, device=self.device)
         ws = {"ab": torch.empty(self.cin, N, **bf),
-              "vb": [torch.empty(C, N, **bf) for _ in range(L + 1)],
-              "z": [torch.empty(C, N, **f32) for _ in range(L if train else 1)],
+              "vb": [torch.empty(C, N, **bf) for _ in range(L + 1 if train or not fused else 2)],
               "Pm": [torch.empty(C * B * m2 * q2, **f32) for _ in range(L if train else 1)],
               "X1p": torch.empty(C * B * m2 * H, **bf),
               "Ym": torch.empty(C * B * q2 * m2, **bf),
               "Z": torch.empty(C * B * H * m2, **bf),
-              "h": torch.empty(self.hidden, N, **f32),
-              "gb": torch.empty(self.hidden, N, **bf),
               "out": torch.empty(self.cout, N, **f32)}
+        if fused:
+            ws["z"] = [torch.empty(C, N, **f32) for _ in range(L - 1 if train else 0)]
+        else:
+            ws.update({"z": [torch.empty(C, N, **f32) for _ in range(L if train else 1)],
+                       "h": torch.empty(self.hidden, N, **f32)})
+        if train or not fused:
+            ws["gb"] = torch.empty(self.hidden, N, **bf)
         if train:
             ws.update({"d": torch.empty(self.cout, N, **f32), "db": torch.empty(self.cout, N, **bf),
-                       "dh": torch.empty(self.hidden, N, **f32), "dhb": torch.empty(self.hidden, N, **bf),
-                       "dv": torch.empty(C, N, **f32),
-                       "dzb": torch.empty(C, N, **bf), "dYm": torch.empty(C * B * q2 * m2, **f32),
+                       "dhb": torch.empty(self.hidden, N, **bf),
+                       "dzb": [torch.empty(C, N, **bf) for _ in range(2 if fused else 1)],
+                       "dYm": torch.empty(C * B * q2 * m2, **f32),
                        "dP": torch.empty(C * B * m2 * q2, **bf),
                        "parts": torch.empty(self.max_splits * max(self.hidden * C, C * C, C * self.cin,
                                                                     self.cout * self.hidden), **f32),
                        "mse": torch.empty(1024, dtype=torch.float64, device=self.device),
                        "rowsum": torch.empty(64 * max(self.hidden, C, self.cout), **f32)})
+            if fused:
+                ws["sums"] = torch.empty(_lib.load().lbgb_fno_layer_parts(max(self.hidden, C)), **f32)
+                # FP32 gradients, where the kernels cannot sum them over the pixels in order
+                flat, rows = (_lib.load().lbgb_fno_layer_sums(*x) for x in ((1, N, 0), (B * H, W, m2)))
+                ws["df"] = None if flat and rows else torch.empty(C if flat else max(self.hidden, C), N, **f32)
+                ws["flat_sums"], ws["row_sums"] = flat, rows
+            else:
+                ws.update({"dh": torch.empty(self.hidden, N, **f32), "dv": torch.empty(C, N, **f32)})
         self._ws[key] = ws
         return ws
 
@@ -292,12 +314,14 @@ class FNO2d:
         N = B * H * W
         ws = self._workspace(B, H, W, train)
         self._shape = (B, H, W)
-        fw, G, iw, _, _ = self.matrices(H, W)
+        _, _, iw, _, _ = self.matrices(H, W)
         C, m = self.width, self.modes
         q2, m2 = 4 * m, 2 * m
         s = self._s()
         pb = self.flat_bf16
         _lib.call("lbgb_fno_to_bf16", a.data_ptr(), ws["ab"].data_ptr(), a.numel(), s)
+        if self._fused(B, H, W):
+            return self._forward_fused(ws, B, H, W, train)
         z0 = ws["z"][0]
         # lifting: v0 = P a + p
         self._gemm(N, C, self.cin, _ptr(ws["ab"]), (1, N, 0), _ptr(pb, self.offsets["P"]), (1, self.cin, 0),
@@ -310,16 +334,7 @@ class FNO2d:
             Pm = ws["Pm"][l] if train else ws["Pm"][0]
             # pointwise branch: z = W_l v
             self._gemm(N, C, C, _ptr(v), (1, N, 0), _ptr(pb, self.offsets["W%d" % l]), (1, C, 0), _ptr(z), (1, N, 0))
-            # spectral branch: W-transform (per channel-sample plane), written as (C, B, 2m, H)
-            self._gemm(H, m2, W, _ptr(v), (W, 1, H * W), _ptr(fw), (1, W, 0), _ptr(ws["X1p"]), (1, H, m2 * H),
-                       batch=C * B, bf16_out=True)
-            # H-transform of every (c, b, kx part) row: P (C, B, 2m, 4m)
-            self._gemm(C * B * m2, q2, H, _ptr(ws["X1p"]), (H, 1, 0), _ptr(G), (1, H, 0), _ptr(Pm), (q2, 1, 0))
-            _lib.call("lbgb_fno_mix", _ptr(Pm), _ptr(pb, self.offsets["Rr%d" % l]), _ptr(pb, self.offsets["Ri%d" % l]),
-                      _ptr(ws["Ym"]), C, C, B, 2 * m, m, s)
-            # inverse along H: Z (C, B, H, 2m)
-            self._gemm(H, m2, q2, _ptr(G), (1, H, 0), _ptr(ws["Ym"]), (m2, 1, q2 * m2), _ptr(ws["Z"]),
-                       (m2, 1, H * m2), batch=C * B, bf16_out=True)
+            self._spectrum(ws, v, l, Pm, B, H, W)
             # inverse along W, added onto the pointwise branch, then bias and
             # activation (in the GEMM's epilogue where the TMA pipeline runs)
             self._gemm_bias_act(C * B * H, W, m2, _ptr(ws["Z"]), (m2, 1), _ptr(iw), m2, _ptr(z), W,
@@ -331,12 +346,54 @@ class FNO2d:
                    (1, C, 0), _ptr(h), (1, N, 0))
         _lib.call("lbgb_fno_bias_act", _ptr(h), _ptr(self.flat, self.offsets["q1b"]), None, None, _ptr(ws["gb"]),
                   self.hidden, N, 1, s)
-        out = ws["out"]
-        self._gemm(N, self.cout, self.hidden, _ptr(ws["gb"]), (1, N, 0), _ptr(pb, self.offsets["Q2"]),
-                   (1, self.hidden, 0), _ptr(out), (1, N, 0))
-        _lib.call("lbgb_fno_bias_act", _ptr(out), _ptr(self.flat, self.offsets["q2b"]), None, None, None,
-                  self.cout, N, 0, s)
-        return out.view(self.cout, B, H, W)
+        self._outputs(ws, N)
+        return ws["out"].view(self.cout, B, H, W)
+
+    def _outputs(self, ws, N):
+        """out = Q2 g + q2b."""
+        out = _ptr(ws["out"])
+        self._gemm(N, self.cout, self.hidden, _ptr(ws["gb"]), (1, N, 0), _ptr(self.flat_bf16, self.offsets["Q2"]),
+                   (1, self.hidden, 0), out, (1, N, 0))
+        _lib.call("lbgb_fno_bias_act", out, _ptr(self.flat, self.offsets["q2b"]), None, None, None, self.cout, N, 0,
+                  self._s())
+
+    def _spectrum(self, ws, v, l, Pm, B, H, W):
+        """The spectral branch of layer l up to its last product: Z (C, B, H, 2m)."""
+        fw, G, _, _, _ = self.matrices(H, W)
+        C, m = self.width, self.modes
+        q2, m2 = 4 * m, 2 * m
+        pb = self.flat_bf16
+        # W-transform (per channel-sample plane), written as (C, B, 2m, H)
+        self._gemm(H, m2, W, _ptr(v), (W, 1, H * W), _ptr(fw), (1, W, 0), _ptr(ws["X1p"]), (1, H, m2 * H),
+                   batch=C * B, bf16_out=True)
+        # H-transform of every (c, b, kx part) row: P (C, B, 2m, 4m)
+        self._gemm(C * B * m2, q2, H, _ptr(ws["X1p"]), (H, 1, 0), _ptr(G), (1, H, 0), _ptr(Pm), (q2, 1, 0))
+        _lib.call("lbgb_fno_mix", _ptr(Pm), _ptr(pb, self.offsets["Rr%d" % l]), _ptr(pb, self.offsets["Ri%d" % l]),
+                  _ptr(ws["Ym"]), C, C, B, 2 * m, m, self._s())
+        # inverse along H
+        self._gemm(H, m2, q2, _ptr(G), (1, H, 0), _ptr(ws["Ym"]), (m2, 1, q2 * m2), _ptr(ws["Z"]),
+                   (m2, 1, H * m2), batch=C * B, bf16_out=True)
+
+    def _forward_fused(self, ws, B, H, W, train):
+        _, _, _, _, iwt = self.matrices(H, W)
+        C, m2, N = self.width, 2 * self.modes, B * H * W
+        s, pb, fl, o = self._s(), self.flat_bf16, self.flat, self.offsets
+        vb = ws["vb"]
+        at = (lambda l: vb[l]) if train else (lambda l: vb[l & 1])
+        _lib.call("lbgb_fno_layer", C, self.cin, 1, N, _ptr(ws["ab"]), _ptr(pb, o["P"]), self.cin, 1, 0, None, None,
+                  _ptr(fl, o["pb"]), 0, None, _ptr(at(0)), s)
+        for l in range(self.layers):
+            last = l == self.layers - 1
+            self._spectrum(ws, at(l), l, ws["Pm"][l if train else 0], B, H, W)
+            _lib.call("lbgb_fno_layer", C, C, B * H, W, _ptr(at(l)), _ptr(pb, o["W%d" % l]), C, 1, m2, _ptr(iwt),
+                      _ptr(ws["Z"]), _ptr(fl, o["b%d" % l]), int(not last),
+                      _ptr(ws["z"][l]) if train and not last else None, _ptr(at(l + 1)), s)
+        _lib.call("lbgb_fno_project", self.hidden, C, 1, N, _ptr(at(self.layers)), _ptr(pb, o["Q1"]),
+                  _ptr(fl, o["q1b"]), self.cout, _ptr(pb, o["Q2"]), _ptr(fl, o["q2b"]),
+                  _ptr(ws["gb"]) if train else None, None if train else _ptr(ws["out"]), s)
+        if train:  # the loss gradient is rounded to BF16: the output in the order of the other engines
+            self._outputs(ws, N)
+        return ws["out"].view(self.cout, B, H, W)
 
     def loss_and_backward(self, a, target, weight=None):
         """Mean squared error of forward(a) against target (cout, B, H, W) and
@@ -347,7 +404,7 @@ class FNO2d:
         out = self.forward(a, train=True)
         B, H, W = self._shape
         N = B * H * W
-        ws = self._ws[(B, H, W, True)]
+        ws = self._ws[(B, H, W, True, self._fused(B, H, W))]
         if target.shape != out.shape or target.dtype != torch.float32 or not target.is_contiguous():
             raise ValueError("target must be a contiguous float32 tensor of shape %s" % (tuple(out.shape),))
         s = self._s()
@@ -366,11 +423,12 @@ class FNO2d:
         return loss
 
     def backward(self, d):
-        """Gradients from d = dLoss/dout (cout, N) FP32 of the last training forward."""
+        """Gradients from d = dLoss/dout (cout, N) FP32 of the last training forward
+        (with the parameters it ran with)."""
         B, H, W = self._shape
         N = B * H * W
-        ws = self._ws[(B, H, W, True)]
-        fw, G, iw, Gt, iwt = self.matrices(H, W)
+        ws = self._ws[(B, H, W, True, self._fused(B, H, W))]
+        fw, _, _, Gt, _ = self.matrices(H, W)
         C, m, hid = self.width, self.modes, self.hidden
         q2, m2 = 4 * m, 2 * m
         s = self._s()
@@ -380,6 +438,9 @@ class FNO2d:
         # out = Q2 g + q2
         self._wgrad(hid, self.cout, N, _ptr(ws["gb"]), _ptr(ws["db"]), _ptr(g, o["Q2"]), 1, hid, ws)
         _lib.call("lbgb_fno_row_sum", _ptr(d), _ptr(g, o["q2b"]), _ptr(ws["rowsum"]), self.cout, N, s)
+        if self._fused(B, H, W):
+            self._backward_fused(ws, B, H, W)
+            return
         dh = ws["dh"]
         self._gemm(N, hid, self.cout, _ptr(ws["db"]), (1, N, 0), _ptr(pb, o["Q2"]), (hid, 1, 0), _ptr(dh), (1, N, 0))
         _lib.call("lbgb_fno_gelu_back", _ptr(dh), _ptr(ws["h"]), _ptr(dh), _ptr(ws["dhb"]), hid * N, s)
@@ -388,7 +449,7 @@ class FNO2d:
         _lib.call("lbgb_fno_row_sum", _ptr(dh), _ptr(g, o["q1b"]), _ptr(ws["rowsum"]), hid, N, s)
         dv = ws["dv"]
         self._gemm(N, C, hid, _ptr(ws["dhb"]), (1, N, 0), _ptr(pb, o["Q1"]), (C, 1, 0), _ptr(dv), (1, N, 0))
-        dzb = ws["dzb"]
+        dzb = ws["dzb"][0]
         for l in reversed(range(self.layers)):
             if l == self.layers - 1:
                 _lib.call("lbgb_fno_to_bf16", _ptr(dv), _ptr(dzb), C * N, s)
@@ -397,14 +458,7 @@ class FNO2d:
             v = ws["vb"][l]
             self._wgrad(C, C, N, _ptr(dzb), _ptr(v), _ptr(g, o["W%d" % l]), C, 1, ws)
             _lib.call("lbgb_fno_row_sum", _ptr(dv), _ptr(g, o["b%d" % l]), _ptr(ws["rowsum"]), C, N, s)
-            # spectral branch, transposed step by step
-            self._gemm(C * B * H, m2, W, _ptr(dzb), (W, 1, 0), _ptr(iwt), (1, W, 0), _ptr(ws["Z"]), (m2, 1, 0),
-                       bf16_out=True)
-            self._gemm(q2, m2, H, _ptr(G), (H, 1, 0), _ptr(ws["Z"]), (m2, 1, H * m2), _ptr(ws["dYm"]),
-                       (m2, 1, q2 * m2), batch=C * B)
-            _lib.call("lbgb_fno_mix_back", _ptr(ws["dYm"]), _ptr(ws["Pm"][l]), _ptr(pb, o["Rr%d" % l]),
-                      _ptr(pb, o["Ri%d" % l]), _ptr(ws["dP"]), _ptr(g, o["Rr%d" % l]), _ptr(g, o["Ri%d" % l]),
-                      C, C, B, 2 * m, m, s)
+            self._spectrum_back(ws, dzb, l, B, H, W)
             self._gemm(C * B * m2, H, q2, _ptr(ws["dP"]), (q2, 1, 0), _ptr(Gt), (1, q2, 0), _ptr(ws["X1p"]),
                        (H, 1, 0), bf16_out=True)
             # pointwise branch: dv = W^T dz, then the spectral branch's input gradient on top
@@ -415,6 +469,48 @@ class FNO2d:
         _lib.call("lbgb_fno_to_bf16", _ptr(dv), _ptr(dzb), C * N, s)
         self._wgrad(C, self.cin, N, _ptr(dzb), _ptr(ws["ab"]), _ptr(g, o["P"]), self.cin, 1, ws)
         _lib.call("lbgb_fno_row_sum", _ptr(dv), _ptr(g, o["pb"]), _ptr(ws["rowsum"]), C, N, s)
+
+    def _spectrum_back(self, ws, dzb, l, B, H, W):
+        """The spectral branch of layer l, transposed step by step, from dz up to
+        the gradient of its H-transform, dP (C, B, 2m, 4m)."""
+        _, G, _, _, iwt = self.matrices(H, W)
+        C, m = self.width, self.modes
+        q2, m2 = 4 * m, 2 * m
+        pb, g, o = self.flat_bf16, self.grad, self.offsets
+        self._gemm(C * B * H, m2, W, _ptr(dzb), (W, 1, 0), _ptr(iwt), (1, W, 0), _ptr(ws["Z"]), (m2, 1, 0),
+                   bf16_out=True)
+        self._gemm(q2, m2, H, _ptr(G), (H, 1, 0), _ptr(ws["Z"]), (m2, 1, H * m2), _ptr(ws["dYm"]),
+                   (m2, 1, q2 * m2), batch=C * B)
+        _lib.call("lbgb_fno_mix_back", _ptr(ws["dYm"]), _ptr(ws["Pm"][l]), _ptr(pb, o["Rr%d" % l]),
+                  _ptr(pb, o["Ri%d" % l]), _ptr(ws["dP"]), _ptr(g, o["Rr%d" % l]), _ptr(g, o["Ri%d" % l]),
+                  C, C, B, 2 * m, m, self._s())
+
+    def _backward_fused(self, ws, B, H, W):
+        fw, _, _, Gt, _ = self.matrices(H, W)
+        C, m, hid, L, N = self.width, self.modes, self.hidden, self.layers, B * H * W
+        q2, m2 = 4 * m, 2 * m
+        s, pb, fl, g, o = self._s(), self.flat_bf16, self.flat, self.grad, self.offsets
+        sums, dhb, vb = _ptr(ws["sums"]), _ptr(ws["dhb"]), ws["vb"]
+        dz, other = ws["dzb"]
+        f32 = _ptr(ws["df"]) if ws["df"] is not None else None
+        flat, rows = None if ws["flat_sums"] else f32, None if ws["row_sums"] else f32
+        _lib.call("lbgb_fno_project_back", hid, C, 1, N, _ptr(vb[L]), _ptr(pb, o["Q1"]), _ptr(fl, o["q1b"]), self.cout,
+                  _ptr(pb, o["Q2"]), _ptr(ws["db"]), dhb, flat, _ptr(g, o["q1b"]), sums, s)
+        self._wgrad(hid, C, N, dhb, _ptr(vb[L]), _ptr(g, o["Q1"]), C, 1, ws)
+        # the gradient of each layer's z, from the last layer's (no activation) down
+        _lib.call("lbgb_fno_layer_back", C, hid, 1, N, dhb, _ptr(pb, o["Q1"]), 1, C, 0, None, None, None, _ptr(dz),
+                  flat, _ptr(g, o["b%d" % (L - 1)] if L else o["pb"]), sums, s)
+        for l in reversed(range(L)):
+            self._wgrad(C, C, N, _ptr(dz), _ptr(vb[l]), _ptr(g, o["W%d" % l]), C, 1, ws)
+            self._spectrum_back(ws, dz, l, B, H, W)
+            # X1 (C, B, H, 2m): the right operand of the last product along W
+            self._gemm(H, m2, q2, _ptr(Gt), (q2, 1, 0), _ptr(ws["dP"]), (1, q2, m2 * q2), _ptr(ws["X1p"]),
+                       (m2, 1, H * m2), batch=C * B, bf16_out=True)
+            _lib.call("lbgb_fno_layer_back", C, C, B * H, W, _ptr(dz), _ptr(pb, o["W%d" % l]), 1, C, m2, _ptr(fw),
+                      _ptr(ws["X1p"]), _ptr(ws["z"][l - 1]) if l else None, _ptr(other), rows,
+                      _ptr(g, o["b%d" % (l - 1)] if l else o["pb"]), sums, s)
+            dz, other = other, dz
+        self._wgrad(C, self.cin, N, _ptr(dz), _ptr(ws["ab"]), _ptr(g, o["P"]), self.cin, 1, ws)
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8, weight_decay=0.0):
         """One Adam step on the FP32 master weights; refreshes the BF16 copy."""
