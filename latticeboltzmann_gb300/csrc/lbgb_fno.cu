@@ -150,84 +150,149 @@ __device__ __forceinline__ void mode_dy(const float *__restrict__ D, int y, int 
     dyi = D[y * m2 + mk + kx] - D[(q + y) * m2 + kx];
 }
 
-__global__ void k_mix_fwd(const float *__restrict__ P, const __nv_bfloat16 *__restrict__ Rr,
+// The mixings are small (19 M complex products each at 16 samples) and bound by the
+// loads of P and dYm, which a warp's modes read from a dozen places.  A thread of
+// mix_fwd and mix_bwd_x takes MIX_G channels of one mode, which share those loads,
+// and the loop is unrolled so that several iterations' loads are in flight: 22 ->
+// 12 and 15 -> 12 us (16 samples, 32 channels, 12 modes).  Each sum keeps its order.
+constexpr int MIX_G = 4;
+
+__global__ void __launch_bounds__(128) k_mix_fwd(const float *__restrict__ P, const __nv_bfloat16 *__restrict__ Rr,
                           const __nv_bfloat16 *__restrict__ Ri, __nv_bfloat16 *__restrict__ Ym, int C, int O, int B,
                           int q, int mk) {
-    const int Q = q * mk;
-    const long long n = (long long)O * B * Q;
+    const int Q = q * mk, groups = (O + MIX_G - 1) / MIX_G;
+    const long long n = (long long)groups * B * Q;
     const long long pcb = 4LL * mk * q;  // P elements per (c, b)
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const int mode = (int)(t % Q), y = mode / mk, kx = mode % mk;
         const int b = (int)((t / Q) % B);
-        const int o = (int)(t / ((long long)Q * B));
-        float ar = 0.f, ai = 0.f;
+        const int o0 = (int)(t / ((long long)Q * B)) * MIX_G;
+        float ar[MIX_G] = {}, ai[MIX_G] = {};
+#pragma unroll 4
         for (int c = 0; c < C; ++c) {
             float xr, xi;
             mode_x(P + ((long long)c * B + b) * pcb, y, kx, q, mk, xr, xi);
-            const long long r = ((long long)c * O + o) * Q + mode;
-            const float rr = __bfloat162float(Rr[r]), ri = __bfloat162float(Ri[r]);
-            ar += xr * rr - xi * ri;
-            ai += xr * ri + xi * rr;
+#pragma unroll
+            for (int i = 0; i < MIX_G; ++i) {
+                const long long r = ((long long)c * O + min(o0 + i, O - 1)) * Q + mode;
+                const float rr = __bfloat162float(Rr[r]), ri = __bfloat162float(Ri[r]);
+                ar[i] += xr * rr - xi * ri;
+                ai[i] += xr * ri + xi * rr;
+            }
         }
-        __nv_bfloat16 *Y = Ym + ((long long)o * B + b) * pcb;
-        const int m2 = 2 * mk;
-        Y[y * m2 + kx] = __float2bfloat16_rn(ar);
-        Y[y * m2 + mk + kx] = __float2bfloat16_rn(ai);
-        Y[(q + y) * m2 + kx] = __float2bfloat16_rn(-ai);
-        Y[(q + y) * m2 + mk + kx] = __float2bfloat16_rn(ar);
+#pragma unroll
+        for (int i = 0; i < MIX_G; ++i) {
+            if (o0 + i >= O) break;
+            __nv_bfloat16 *Y = Ym + ((long long)(o0 + i) * B + b) * pcb;
+            const int m2 = 2 * mk;
+            Y[y * m2 + kx] = __float2bfloat16_rn(ar[i]);
+            Y[y * m2 + mk + kx] = __float2bfloat16_rn(ai[i]);
+            Y[(q + y) * m2 + kx] = __float2bfloat16_rn(-ai[i]);
+            Y[(q + y) * m2 + mk + kx] = __float2bfloat16_rn(ar[i]);
+        }
     }
 }
 
 // Gradient with respect to the inputs: dYm (O, B, 2q, 2mk) FP32 -> dP (C, B, 2mk, 2q) BF16
-__global__ void k_mix_bwd_x(const float *__restrict__ dYm, const __nv_bfloat16 *__restrict__ Rr,
+__global__ void __launch_bounds__(128) k_mix_bwd_x(const float *__restrict__ dYm, const __nv_bfloat16 *__restrict__ Rr,
                             const __nv_bfloat16 *__restrict__ Ri, __nv_bfloat16 *__restrict__ dP, int C, int O, int B,
                             int q, int mk) {
-    const int Q = q * mk;
-    const long long n = (long long)C * B * Q;
+    const int Q = q * mk, groups = (C + MIX_G - 1) / MIX_G;
+    const long long n = (long long)groups * B * Q;
     const long long pcb = 4LL * mk * q;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const int mode = (int)(t % Q), y = mode / mk, kx = mode % mk;
         const int b = (int)((t / Q) % B);
-        const int c = (int)(t / ((long long)Q * B));
-        float ar = 0.f, ai = 0.f;
+        const int c0 = (int)(t / ((long long)Q * B)) * MIX_G;
+        float ar[MIX_G] = {}, ai[MIX_G] = {};
+#pragma unroll 4
         for (int o = 0; o < O; ++o) {
             float gr, gi;
             mode_dy(dYm + ((long long)o * B + b) * pcb, y, kx, q, mk, gr, gi);
-            const long long r = ((long long)c * O + o) * Q + mode;
-            const float rr = __bfloat162float(Rr[r]), ri = __bfloat162float(Ri[r]);
-            ar += gr * rr + gi * ri;
-            ai += -gr * ri + gi * rr;
+#pragma unroll
+            for (int i = 0; i < MIX_G; ++i) {
+                const long long r = ((long long)min(c0 + i, C - 1) * O + o) * Q + mode;
+                const float rr = __bfloat162float(Rr[r]), ri = __bfloat162float(Ri[r]);
+                ar[i] += gr * rr + gi * ri;
+                ai[i] += -gr * ri + gi * rr;
+            }
         }
-        __nv_bfloat16 *D = dP + ((long long)c * B + b) * pcb;
-        const int q2 = 2 * q;
-        D[kx * q2 + y] = __float2bfloat16_rn(ar);
-        D[(mk + kx) * q2 + q + y] = __float2bfloat16_rn(ar);
-        D[(mk + kx) * q2 + y] = __float2bfloat16_rn(ai);
-        D[kx * q2 + q + y] = __float2bfloat16_rn(-ai);
+#pragma unroll
+        for (int i = 0; i < MIX_G; ++i) {
+            if (c0 + i >= C) break;
+            __nv_bfloat16 *D = dP + ((long long)(c0 + i) * B + b) * pcb;
+            const int q2 = 2 * q;
+            D[kx * q2 + y] = __float2bfloat16_rn(ar[i]);
+            D[(mk + kx) * q2 + q + y] = __float2bfloat16_rn(ar[i]);
+            D[(mk + kx) * q2 + y] = __float2bfloat16_rn(ai[i]);
+            D[kx * q2 + q + y] = __float2bfloat16_rn(-ai[i]);
+        }
     }
 }
 
-// Gradient with respect to the weights: dR (C, O, q, mk) FP32, summed over the batch
+// Gradient with respect to the weights: dR (C, O, q, mk) FP32, summed over the batch.
+// A block takes one ky, up to MIXR_K kx, MIXR_C x MIXR_O channels: their x and dy
+// go through shared memory MIXR_B samples at a time, since every (c, o) pair that
+// reads them from L2 reads 32-byte sectors for 4-byte values (50 us; here 29).
+constexpr int MIXR_K = 16, MIXR_C = 4, MIXR_O = 32, MIXR_B = 8, MIXR_T = 16;
+
 __global__ void k_mix_bwd_r(const float *__restrict__ dYm, const float *__restrict__ P, float *__restrict__ dRr,
-                            float *__restrict__ dRi, int C, int O, int B, int q, int mk) {
-    const int Q = q * mk;
-    const long long n = (long long)C * O * Q;
+                            float *__restrict__ dRi, int C, int O, int B, int q, int mk, int kt) {
+    extern __shared__ float2 mix_sm[];  // x [MIXR_C][MIXR_B][kt], then dy [MIXR_O][MIXR_B][kt]
+    float2 *sx = mix_sm, *sg = mix_sm + MIXR_C * MIXR_B * kt;
+    const int Q = q * mk, y = blockIdx.x % q, k0 = blockIdx.x / q * kt;
+    const int o0 = blockIdx.y * MIXR_O, c0 = blockIdx.z * MIXR_C;
     const long long pcb = 4LL * mk * q;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int mode = (int)(t % Q), y = mode / mk, kx = mode % mk;
-        const int o = (int)((t / Q) % O);
-        const int c = (int)(t / ((long long)Q * O));
-        float ar = 0.f, ai = 0.f;
-        for (int b = 0; b < B; ++b) {
-            float gr, gi, xr, xi;
-            mode_dy(dYm + ((long long)o * B + b) * pcb, y, kx, q, mk, gr, gi);
-            mode_x(P + ((long long)c * B + b) * pcb, y, kx, q, mk, xr, xi);
-            ar += gr * xr + gi * xi;
-            ai += -gr * xi + gi * xr;
+    const int k = threadIdx.x % kt, og = threadIdx.x / kt;  // this thread's kx and every MIXR_T-th o from og
+    constexpr int NO = MIXR_O / MIXR_T;
+    float ar[MIXR_C][NO] = {}, ai[MIXR_C][NO] = {};
+    for (int b0 = 0; b0 < B; b0 += MIXR_B) {
+        const int nb = min(MIXR_B, B - b0);
+#pragma unroll 3
+        for (int e = og; e < (MIXR_C + MIXR_O) * nb; e += MIXR_T) {
+            const int ch = e / nb, b = e - ch * nb;
+            const bool is_x = ch < MIXR_C;
+            const int c = is_x ? c0 + ch : o0 + ch - MIXR_C;
+            float2 v = make_float2(0.f, 0.f);
+            if (k0 + k < mk && c < (is_x ? C : O)) {
+                if (is_x)
+                    mode_x(P + ((long long)c * B + b0 + b) * pcb, y, k0 + k, q, mk, v.x, v.y);
+                else
+                    mode_dy(dYm + ((long long)c * B + b0 + b) * pcb, y, k0 + k, q, mk, v.x, v.y);
+            }
+            (is_x ? sx + ch * MIXR_B * kt : sg + (ch - MIXR_C) * MIXR_B * kt)[b * kt + k] = v;
         }
-        dRr[t] = ar;
-        dRi[t] = ai;
+        __syncthreads();
+        for (int b = 0; b < nb; ++b) {
+            float2 g[NO];
+#pragma unroll
+            for (int i = 0; i < NO; ++i) g[i] = sg[((og + i * MIXR_T) * MIXR_B + b) * kt + k];
+#pragma unroll
+            for (int h = 0; h < MIXR_C; ++h) {
+                const float2 x = sx[(h * MIXR_B + b) * kt + k];
+                const float xr = x.x, xi = x.y;
+#pragma unroll
+                for (int i = 0; i < NO; ++i) {
+                    const float gr = g[i].x, gi = g[i].y;
+                    ar[h][i] += gr * xr + gi * xi;
+                    ai[h][i] += -gr * xi + gi * xr;
+                }
+            }
+        }
+        __syncthreads();
     }
+    if (k0 + k >= mk) return;
+#pragma unroll
+    for (int h = 0; h < MIXR_C; ++h)
+#pragma unroll
+        for (int i = 0; i < NO; ++i) {
+            const int c = c0 + h, o = o0 + og + i * MIXR_T;
+            if (c < C && o < O) {
+                const long long r = ((long long)c * O + o) * Q + y * mk + k0 + k;
+                dRr[r] = ar[h][i];
+                dRi[r] = ai[h][i];
+            }
+        }
 }
 
 // mean squared error: partial sums per block into part[], and d = 2 (y - t) / n
@@ -295,7 +360,8 @@ __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float
 // (x, y) adds the splits s = y, y + SUM_GROUPS, ... (loads coalesced over x),
 // then the group sums are added in the fixed order y = 0, 1, ...  (One
 // thread per output walking all S splits left the few hundred threads of a
-// weight gradient waiting on S dependent additions.)
+// weight gradient waiting on S dependent additions.)  The loads of 16 splits are
+// in flight together: 20 -> 11 us at 1024 splits of 1024 outputs against 4.
 constexpr int SUM_GROUPS = 8;
 __global__ void __launch_bounds__(32 * SUM_GROUPS)
 k_sum_splits(const float *__restrict__ parts, float *__restrict__ out, int S, long long n, float beta) {
@@ -303,7 +369,7 @@ k_sum_splits(const float *__restrict__ parts, float *__restrict__ out, int S, lo
     const long long i = blockIdx.x * 32ll + threadIdx.x;
     float acc = 0.f;
     if (i < n) {
-#pragma unroll 4
+#pragma unroll 16
         for (int s = threadIdx.y; s < S; s += SUM_GROUPS) acc += parts[(long long)s * n + i];
     }
     part[threadIdx.y][threadIdx.x] = acc;
@@ -393,9 +459,9 @@ extern "C" int lbgb_fno_row_sum(const float *dy, float *db, float *partials, int
 
 extern "C" int lbgb_fno_mix(const float *P, const void *Rr, const void *Ri, void *Ym, int C, int O, int B, int q,
                             int mk, void *stream) {
-    const long long n = (long long)O * B * q * mk;
+    const long long n = (long long)((O + MIX_G - 1) / MIX_G) * B * q * mk;
     if (n <= 0 || C <= 0) return LBGB_OK;
-    k_mix_fwd<<<blocks_for(n), 256, 0, (cudaStream_t)stream>>>(P, static_cast<const __nv_bfloat16 *>(Rr),
+    k_mix_fwd<<<blocks_for(2 * n), 128, 0, (cudaStream_t)stream>>>(P, static_cast<const __nv_bfloat16 *>(Rr),
                                                                static_cast<const __nv_bfloat16 *>(Ri),
                                                                static_cast<__nv_bfloat16 *>(Ym), C, O, B, q, mk);
     return check_launch("k_mix_fwd");
@@ -405,12 +471,18 @@ extern "C" int lbgb_fno_mix_back(const float *dYm, const float *P, const void *R
                                  float *dRr, float *dRi, int C, int O, int B, int q, int mk, void *stream) {
     if (C <= 0 || O <= 0 || B <= 0 || q <= 0 || mk <= 0) return LBGB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    k_mix_bwd_x<<<blocks_for((long long)C * B * q * mk), 256, 0, s>>>(
+    k_mix_bwd_x<<<blocks_for(2ll * ((C + MIX_G - 1) / MIX_G) * B * q * mk), 128, 0, s>>>(
         dYm, static_cast<const __nv_bfloat16 *>(Rr), static_cast<const __nv_bfloat16 *>(Ri),
         static_cast<__nv_bfloat16 *>(dP), C, O, B, q, mk);
     int rc = check_launch("k_mix_bwd_x");
     if (rc) return rc;
-    k_mix_bwd_r<<<blocks_for((long long)C * O * q * mk), 256, 0, s>>>(dYm, P, dRr, dRi, C, O, B, q, mk);
+    const int kt = mk < MIXR_K ? mk : MIXR_K, ot = (O + MIXR_O - 1) / MIXR_O, ct = (C + MIXR_C - 1) / MIXR_C;
+    if (ot > 65535 || ct > 65535 || (long long)q * ((mk + kt - 1) / kt) > 2147483647ll) {
+        set_error("lbgb_fno_mix_back: too many channels or modes");
+        return LBGB_EINVAL;
+    }
+    const size_t smem = sizeof(float2) * (MIXR_C + MIXR_O) * MIXR_B * kt;
+    k_mix_bwd_r<<<dim3(q * ((mk + kt - 1) / kt), ot, ct), kt * MIXR_T, smem, s>>>(dYm, P, dRr, dRi, C, O, B, q, mk, kt);
     return check_launch("k_mix_bwd_r");
 }
 
