@@ -1075,7 +1075,7 @@ extern "C" int lbgb_fno_layer_back(int n, int k1, int rows, int w, const void *x
 
 extern "C" int lbgb_fno_project(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
                                 int cout, const void *q2, const float *q2b, void *g, float *out, void *stream) {
-    if (!x || !q1 || !q1b || (!g && !out) || (out && (!q2 || !q2b)) || (g && !aligned(g, 4))) {
+    if (!x || !q1 || !q1b || (!g && !out) || (out && (!q2 || !q2b)) || (g && !aligned(g, 16))) {
         set_error("lbgb_fno_project: null or misaligned operand");
         return LBGB_EINVAL;
     }
@@ -1084,13 +1084,17 @@ extern "C" int lbgb_fno_project(int n, int k1, int rows, int w, const void *x, c
     a.b1 = static_cast<const __nv_bfloat16 *>(q1), a.b1_ns = k1, a.b1_ks = 1;
     a.bias = q1b, a.cout = cout, a.q2 = static_cast<const __nv_bfloat16 *>(q2), a.q2b = q2b;
     a.v = static_cast<__nv_bfloat16 *>(g), a.out = out;
+    if (g) {
+        const int rc = launch_layer<HIDDEN>(a, x, nullptr, nullptr, nullptr, (cudaStream_t)stream, "lbgb_fno_project");
+        if (rc || !out) return rc;
+    }
     return launch_layer<PROJECT>(a, x, nullptr, nullptr, nullptr, (cudaStream_t)stream, "lbgb_fno_project");
 }
 
 extern "C" int lbgb_fno_project_back(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
                                      int cout, const void *q2, const void *d, void *dh, float *f32, float *sums,
                                      float *parts, void *stream) {
-    if (!x || !q1 || !q1b || !q2 || !d || !dh || !sums || !parts || cout < 1 || !aligned(dh, 4)) {
+    if (!x || !q1 || !q1b || !q2 || !d || !dh || !sums || !parts || cout < 1 || !aligned(dh, 16) || (f32 && !aligned(f32, 16))) {
         set_error("lbgb_fno_project_back: null or misaligned operand");
         return LBGB_EINVAL;
     }

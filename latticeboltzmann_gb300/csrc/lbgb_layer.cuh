@@ -1,5 +1,5 @@
 // The surrogate's pointwise layers with everything that follows them up to the
-// next product: one persistent tcgen05 kernel, four epilogues.
+// next product: one persistent tcgen05 kernel, five epilogues.
 //
 // Activations are channel-major, (channels, rows * W): a row is one grid line
 // of one sample.
@@ -17,20 +17,20 @@
 //             BF16; a2 are cosines over w, b2 a row's modes
 //   BACK      dz = (D2 + D1) gelu'(z) (or D2 + D1) BF16, and its sum over the
 //             pixels; a2, b2 as in LAYER
-//   PROJECT   g = gelu(D1 + bias) BF16, and out = Q2 g + q2b where a pass wants
-//             nothing else: the hidden layer's FP32 values are never stored
+//   HIDDEN    g = gelu(D1 + bias) BF16 (training)
+//   PROJECT   out = Q2 g + q2b of the same g, which is not stored (inference)
 //   PROJECT_BACK  D1 + bias computed again (the product reads 1/8 of the bytes
 //             that the stored values would be), D2 = d Q2 (a2 is d, b2 is Q2),
 //             dh = D2 gelu'(D1 + bias) BF16, and its sum over the pixels
 //
 // What they cannot do without is the activations in and out once.  16 x 256^2, 32
 // channels (us; the passes replaced -> here, and the bytes at the copy rate):
-// LAYER 178 -> 52 (43), BACK 212 -> 79 (43), PROJECT 325 -> 121 (50),
-// PROJECT_BACK 462 -> 210 (50).  The projections are bound by the epilogue's
-// instructions (128 channels a pixel).  BACK takes z through shared memory with
-// the other operands: loaded by the lanes themselves it waited out DRAM's
-// latency at every tile (+22).  The order of the sums costs 14 and 70 against
-// sums kept in each lane.
+// LAYER 178 -> 52 (43), BACK 212 -> 79 (43), HIDDEN 325 -> 93 (50), PROJECT_BACK
+// 462 -> 145 (50).  The last two are bound by the epilogue's instructions (128
+// channels a pixel).  BACK takes z through shared memory with the other operands:
+// loaded by the lanes themselves it waited out DRAM's latency at every tile (+22).
+// With lane = pixel, HIDDEN took 121 and PROJECT_BACK 210 (the ordered sums through
+// shared memory, 64-bit address steps and a bias load per value).
 //
 //  * warp 0, one thread: TMA producer; a stage holds one tile's operands (x and
 //    a2 pixel-major boxes of 64 pixels x up to 64 k, b2 k-major; 128-byte
@@ -39,14 +39,16 @@
 //    shared memory for all tiles, in the same swizzled layout (and so does Q2).
 //  * EG groups of four warps: epilogue; lane = pixel, register = channel.  A
 //    channel's stores are 32 neighbouring pixels.  The groups split a tile's
-//    channels (LAYER, BACK, PROJECT_BACK) or take tiles in turn (PROJECT: a
-//    pixel's outputs need all its hidden channels).
+//    channels (LAYER, BACK) or take tiles in turn (PROJECT: a pixel's outputs need
+//    all its hidden channels).  HIDDEN and PROJECT_BACK (128 channels) exchange the
+//    operands: lane = channel, register = pixel, so that bias, sums and packing
+//    stay within a lane and a store is 8 pixels.
 // Waits are bounded as in the GEMM pipeline.
 #pragma once
 
 namespace lbgb {
 
-enum { LAYER = 0, BACK = 1, PROJECT = 2, PROJECT_BACK = 3 };
+enum { LAYER = 0, BACK = 1, PROJECT = 2, PROJECT_BACK = 3, HIDDEN = 4 };
 
 struct LayerArgs {
     int n, k1, k2;                 // channels out, channels in, modes (0: no second product)
@@ -75,18 +77,19 @@ struct LayerArgs {
 // them the tiles of 128 pixels, 1024 apart, in order; where the tiles do not
 // fall so (layer_chunk), the FP32 values are stored and summed by k_row_sum.
 constexpr int SUM_CHUNKS = 64;
-constexpr int LAYER_SMEM = 108 * 1024;  // operands of a CTA: two CTAs fit an SM
 
 template <int MODE> struct LayerShape {
-    static constexpr int NT = MODE == PROJECT || MODE == PROJECT_BACK ? 128 : 32;
+    static constexpr bool FLIP = MODE == PROJECT_BACK || MODE == HIDDEN;  // accumulator lanes are channels
+    static constexpr int NT = MODE == PROJECT || FLIP ? 128 : 32;
     static constexpr int EG = MODE == PROJECT_BACK ? 4 : 2;      // epilogue groups of four warps
     static constexpr int CTAS = MODE == PROJECT_BACK ? 1 : 2;
     static constexpr int THREADS = 64 + EG * 128;
     static constexpr bool TURNS = MODE == PROJECT;               // groups take tiles in turn
-    static constexpr int COLS = TURNS ? NT : NT / EG;            // channels per group
-    static constexpr bool TWO = MODE != PROJECT;                 // two products
+    static constexpr int COLS = TURNS ? NT : NT / EG;            // accumulator columns per group
+    static constexpr bool TWO = MODE != PROJECT && MODE != HIDDEN;  // two products
     static constexpr int TMEM = 2 * NT * (TWO ? 2 : 1);          // two buffers
-    static constexpr int CH = MODE == PROJECT_BACK ? 8 : 16;     // channels per TMEM load
+    static constexpr int CH = 16;                                // columns per TMEM load
+    static constexpr int SMEM = (CTAS == 1 ? 200 : 108) * 1024;  // shared memory of a CTA's operands
 };
 
 // b1 in the K-major 128-byte-swizzled layout: 64-k blocks of NT rows x 128 bytes
@@ -103,7 +106,26 @@ __device__ __forceinline__ void store_pair(__nv_bfloat16 *v, int lane, bool in, 
     if (in) *reinterpret_cast<__nv_bfloat162 *>(v) = w;
 }
 
-// 16 or 8 consecutive accumulator columns of this warp's 32 lanes (to be waited for)
+// Stores 64 bytes of each of 32 rows, `stride` bytes apart, that the lanes hold
+// (lane = row): turned in shared memory (2 KB a warp, 16-byte units swizzled) so
+// that four lanes write a row's 64 bytes.  Written row by row from the lanes, 32
+// lines an instruction, HIDDEN took 347 us and PROJECT_BACK 425.
+__device__ __forceinline__ void store_rows(uint4 *buf, const uint4 (&w)[4], int lane, void *to, long long stride,
+                                           int rows, int units) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) buf[lane * 4 + (i ^ (lane >> 1 & 3))] = w[i];
+    __syncwarp();
+    const int u = lane & 3;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = lane / 4 + 8 * i;
+        const uint4 x = buf[r * 4 + (u ^ (r >> 1 & 3))];
+        if (r < rows && u < units) *reinterpret_cast<uint4 *>(static_cast<char *>(to) + r * stride + u * 16) = x;
+    }
+    __syncwarp();
+}
+
+// 16 consecutive accumulator columns of this warp's 32 lanes (to be waited for)
 __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -111,11 +133,6 @@ __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&v)[16]) {
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
-}
-__device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&v)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(taddr));
 }
 
 // Calls tile(p0, end) for this CTA's tiles in order, pixels [p0, min(p0 + 128, end)),
@@ -190,7 +207,7 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         if (MODE == PROJECT) {
             float q[4] = {0.f, 0.f, 0.f, 0.f};
             for (int o = 0; o < 4; ++o)
-                if (a.out && o < a.cout && c < a.n) q[o] = __bfloat162float(a.q2[(long long)o * a.n + c]);
+                if (o < a.cout && c < a.n) q[o] = __bfloat162float(a.q2[(long long)o * a.n + c]);
             s_q2[c] = make_float4(q[0], q[1], q[2], q[3]);
         }
     }
@@ -234,11 +251,13 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(TC_M, NT) | (1u << 15);  // bit 15: A MN-major
+            // bit 15: A MN-major, bit 16: B MN-major (the pixels' operand)
+            constexpr uint32_t idesc = umma_idesc_bf16(TC_M, NT) | (S::FLIP ? 1u << 16 : 1u << 15);
             int it = 0;
             uint64_t *last = nullptr;
             uint32_t last_ph = 0;
-            auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t acc) {
+            auto mma = [&](uint32_t d, uint64_t pixels, uint64_t channels, uint32_t acc) {
+                const uint64_t da = S::FLIP ? channels : pixels, db = S::FLIP ? pixels : channels;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.u32 p, %4, 0;\n\t"
@@ -288,9 +307,9 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         const int q = warp & 3, group = (warp - 2) >> 2;
         const int col0 = S::TURNS ? 0 : group * COLS;
         constexpr bool SUMS = MODE == BACK || MODE == PROJECT_BACK;
-        // SUMS: this lane adds four pixels (quad lane % 8 of the warp's 32) of
+        // SUMS (BACK): this lane adds four pixels (quad lane % 8 of the warp's 32) of
         // channels lane / 8 + 4 i, from the warp's block of CH x 32 values
-        [[maybe_unused]] float *turn = reinterpret_cast<float *>(dsm + a.turn_at) + (warp - 2) * CH * 32;
+        [[maybe_unused]] float *turn = reinterpret_cast<float *>(dsm + a.turn_at) + (warp - 2) * 512;
         float acc[SUMS ? COLS / 4 : 1] = {};
         int it = 0;
         walk_tiles(a, [&](int p0, int end) {
@@ -310,10 +329,59 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float out[4] = {0.f, 0.f, 0.f, 0.f};
             // MODE's arithmetic on this warp's channels.  ACT: with gelu;
-            // KEEP: LAYER stores z, PROJECT computes out, BACK and PROJECT_BACK store
-            // FP32 values instead of adding them
+            // KEEP: LAYER stores z, BACK and PROJECT_BACK store FP32 values instead of
+            // adding them
             auto columns = [&](auto act, auto keep) {
                 [[maybe_unused]] constexpr bool ACT = decltype(act)::value, KEEP = decltype(keep)::value;
+                if constexpr (S::FLIP) {
+                    // lane = channel, column = pixel, 32 pixels at a time
+                    const int c = q * 32;
+                    const float b = s_bias[c + lane];
+                    const int first = p0 + col0, n = end - first;  // whole groups of 8 pixels
+#pragma unroll
+                    for (int c0 = 0; c0 < COLS; c0 += 32) {
+                        if (c0 >= n) break;
+                        uint4 w[4];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t d1[CH];
+                            [[maybe_unused]] uint32_t d2[CH];
+                            const uint32_t at =
+                                tmem + ((uint32_t)c << 16) + (uint32_t)(buf * (S::TMEM / 2) + col0 + c0 + h * CH);
+                            tc_ld(at, d1);
+                            if constexpr (S::TWO) tc_ld(at + NT, d2);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            float y[CH];
+#pragma unroll
+                            for (int e = 0; e < CH; ++e) {
+                                const float x = __uint_as_float(d1[e]) + b;
+                                if constexpr (MODE == PROJECT_BACK)
+                                    y[e] = __uint_as_float(d2[e]) * gelu_df(x);
+                                else
+                                    y[e] = gelu_f(x);
+                                if constexpr (SUMS && !KEEP)
+                                    if (c0 + h * CH + e / 8 * 8 < n) acc[(c0 + h * CH + e) / 4] += y[e];
+                            }
+                            if constexpr (SUMS && KEEP) {
+                                uint4 f[4];
+                                memcpy(f, y, sizeof(f));
+                                store_rows(reinterpret_cast<uint4 *>(turn), f, lane, a.f32 + c * N + first + c0 + h * CH, N * 4,
+                                           a.n - c, (n - c0 - h * CH) / 4);
+                            }
+                            uint32_t two[CH / 2];
+#pragma unroll
+                            for (int e = 0; e < CH / 2; ++e) {
+                                const __nv_bfloat162 z2 = __floats2bfloat162_rn(y[2 * e], y[2 * e + 1]);
+                                memcpy(two + e, &z2, 4);
+                            }
+                            w[2 * h] = make_uint4(two[0], two[1], two[2], two[3]);
+                            w[2 * h + 1] = make_uint4(two[4], two[5], two[6], two[7]);
+                        }
+                        store_rows(reinterpret_cast<uint4 *>(turn), w, lane, a.v + c * N + first + c0, N * 2, a.n - c,
+                                   (n - c0) / 8);
+                    }
+                    return;
+                }
                 __nv_bfloat16 *v = a.v + (col0 + (lane & 1)) * N + (p & ~1ll);
                 [[maybe_unused]] float *z = (SUMS ? a.f32 : a.z) + col0 * N + p;
                 [[maybe_unused]] const float *zs = reinterpret_cast<const float *>(dsm + (size_t)st * a.stage_bytes + z_at) +
@@ -337,19 +405,16 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
                             float x = __uint_as_float(d1[j + e]);
                             if constexpr (MODE == LAYER || MODE == BACK) x = __uint_as_float(d2[j + e]) + x;
                             if constexpr (MODE != BACK) x += s_bias[col0 + c];
-                            if constexpr (MODE == BACK) {
+                            if constexpr (MODE == BACK)
                                 y[e] = ACT ? x * gelu_df(zs[c * TC_M]) : x;
-                            } else if constexpr (MODE == PROJECT_BACK) {
-                                y[e] = __uint_as_float(d2[j + e]) * gelu_df(x);
-                            } else {
+                            else
                                 y[e] = ACT ? gelu_f(x) : x;
-                            }
                             if constexpr (SUMS && !KEEP) turn[(j + e) * 32 + lane] = in ? y[e] : 0.f;
                             if constexpr ((MODE == LAYER || SUMS) && KEEP) {
                                 if (in) *z = SUMS ? y[e] : x;
                                 z += N;
                             }
-                            if constexpr (MODE == PROJECT && KEEP) {
+                            if constexpr (MODE == PROJECT) {
                                 const float g = __bfloat162float(__float2bfloat16_rn(y[e]));
                                 const float4 w = s_q2[col0 + c];
                                 out[0] += g * w.x;
@@ -358,7 +423,7 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
                                 out[3] += g * w.w;
                             }
                         }
-                        if (MODE != PROJECT || a.v) store_pair(v, lane, in, y[0], y[1]);
+                        if constexpr (MODE != PROJECT) store_pair(v, lane, in, y[0], y[1]);
                         v += 2 * N;
                     }
                     if constexpr (SUMS && !KEEP) {
@@ -377,7 +442,7 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
                 }
             };
             using std::bool_constant;
-            if (p0 + q * 32 < end) {
+            if (p0 + (S::FLIP ? col0 : q * 32) < end) {
                 if constexpr (MODE == LAYER) {
                     if (a.act)
                         a.z ? columns(bool_constant<true>(), bool_constant<true>())
@@ -392,12 +457,11 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
                     else
                         a.f32 ? columns(bool_constant<false>(), bool_constant<true>())
                               : columns(bool_constant<false>(), bool_constant<false>());
-                } else if constexpr (MODE == PROJECT) {
-                    a.out ? columns(bool_constant<true>(), bool_constant<true>())
-                          : columns(bool_constant<true>(), bool_constant<false>());
-                } else {
+                } else if constexpr (MODE == PROJECT_BACK) {
                     a.f32 ? columns(bool_constant<true>(), bool_constant<true>())
                           : columns(bool_constant<true>(), bool_constant<false>());
+                } else {
+                    columns(bool_constant<true>(), bool_constant<false>());
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -406,7 +470,7 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
             if constexpr (MODE == PROJECT) {
 #pragma unroll
                 for (int o = 0; o < 4; ++o)
-                    if (a.out && o < a.cout && in) a.out[o * N + p] = out[o] + a.q2b[o];
+                    if (o < a.cout && in) a.out[o * N + p] = out[o] + a.q2b[o];
             }
             ++it;
             return true;
@@ -414,8 +478,9 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
             if constexpr (SUMS) {
 #pragma unroll
                 for (int i = 0; i < COLS / 4; ++i) {
-                    const int c = col0 + lane / 8 + 4 * i;
-                    if (c < a.n) a.parts[((long long)c * SUM_CHUNKS + (u >> 3)) * 256 + (u & 7) * 32 + q * 8 + lane % 8] = acc[i];
+                    const int c = S::FLIP ? q * 32 + lane : col0 + lane / 8 + 4 * i;
+                    const int quad = S::FLIP ? col0 / 4 + i : q * 8 + lane % 8;
+                    if (c < a.n) a.parts[((long long)c * SUM_CHUNKS + (u >> 3)) * 256 + (u & 7) * 32 + quad] = acc[i];
                     acc[i] = 0.f;
                 }
             }
@@ -518,9 +583,13 @@ static int launch_layer(LayerArgs a, const void *x, const void *a2, const void *
     a.stage_bytes = kb1 * 2 * a.box1 * 128 + (a.k2 ? 2 * a.box2 * 128 + (RESIDENT2 ? 0 : S::NT * 128) : 0) +
                     (MODE == BACK && a.z ? S::NT * TC_M * 4 : 0);
     const int b1_bytes = S::NT * kb1 * 128 + (RESIDENT2 ? S::NT * 128 : 0);
-    const int turn_bytes = sums && !a.f32 ? S::EG * 4 * S::CH * 32 * 4 : 0;
-    a.stages = (LAYER_SMEM - b1_bytes - turn_bytes) / a.stage_bytes;
+    const int turn_bytes = S::FLIP || (MODE == BACK && !a.f32) ? S::EG * 4 * 2048 : 0;  // 2 KB a warp
+    a.stages = (S::SMEM - b1_bytes - turn_bytes) / a.stage_bytes;
     if (a.stages > 4) a.stages = 4;
+    if (a.stages < 1) {
+        set_error("%s: no room for the operands of a tile", what);
+        return LBGB_EINVAL;
+    }
     a.turn_at = a.stages * a.stage_bytes + b1_bytes;
     const int smem = a.turn_at + turn_bytes;
     a.chunk = sums && !a.f32 ? layer_chunk(a.rows, a.W, MODE == BACK && a.k2) : 0;
@@ -544,7 +613,7 @@ static int launch_layer(LayerArgs a, const void *x, const void *a2, const void *
     const int dev = current_device();
     if (!attr[dev].load(std::memory_order_acquire)) {
         std::lock_guard<std::mutex> lock(setup_mutex());
-        const cudaError_t e = cudaFuncSetAttribute(k_layer<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(k_layer<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
         if (e != cudaSuccess) {
             set_error("%s: cannot reserve shared memory: %s", what, cudaGetErrorString(e));
             return LBGB_ECUDA;
