@@ -215,7 +215,7 @@ __device__ __forceinline__ void ip_stream_tile(const typename Codec<DT>::raw *s,
 // halo into shared memory, then the streamed tile back over itself.
 template <int DT, int BC>
 __global__ void __launch_bounds__(IP_THREADS, 2)
-k_ip_stream(typename Codec<DT>::raw *f, const typename Codec<DT>::raw *__restrict__ ws, int nx, int ny,
+k_ip_stream(typename Codec<DT>::raw *f, const typename Codec<DT>::raw *__restrict__ ws, int nx, int ny, int,
             typename Codec<DT>::real u0) {
     using raw = typename Codec<DT>::raw;
     using G = IpGeom<raw>;
@@ -242,7 +242,7 @@ k_ip_stream(typename Codec<DT>::raw *f, const typename Codec<DT>::raw *__restric
 
 // Pipelined form for rows of whole 16-byte vectors (16-byte aligned f, ny a
 // multiple of the vector width): one persistent block per SM with two
-// stages, streaming runs of IP_RUN consecutive tiles along y, each run in
+// stages, streaming runs of up to IP_RUN consecutive tiles along y, each run in
 // order.  While a tile is streamed out of one stage, the next tile's interior
 // is on its way into the other (16-byte cp.async, one group per tile) and its
 // halo values into registers, so the SM's loads and stores overlap instead of
@@ -292,9 +292,11 @@ __device__ __forceinline__ const raw *ip_run_halo(int i, const IpTile &T, int sg
     return ws + L.col_off + (((long long)ulo * 2 + 1) * 3 + j) * nx + T.a + r;
 }
 
-template <int DT, int BC>
+// RUN: the run length, or 0: `run` (a run of IP_RUN known to the compiler is 1 %
+// faster at 4096^2)
+template <int DT, int BC, int RUN>
 __global__ void __launch_bounds__(IPP_THREADS, 1)
-k_ip_stream_pipe(typename Codec<DT>::raw *f, const typename Codec<DT>::raw *__restrict__ ws, int nx, int ny,
+k_ip_stream_pipe(typename Codec<DT>::raw *f, const typename Codec<DT>::raw *__restrict__ ws, int nx, int ny, int run,
                  typename Codec<DT>::real u0) {
     using raw = typename Codec<DT>::raw;
     using G = IpGeom<raw>;
@@ -304,7 +306,7 @@ k_ip_stream_pipe(typename Codec<DT>::raw *f, const typename Codec<DT>::raw *__re
     static_assert(9 * IP_TX * G::VPR % IPP_THREADS == 0, "full tiles split evenly over the threads");
     extern __shared__ __align__(16) unsigned char ip_smem[];
     raw *sm = reinterpret_cast<raw *>(ip_smem);
-    const IpLayout L = ip_layout<raw>(nx, ny, IP_RUN);
+    const IpLayout L = ip_layout<raw>(nx, ny, RUN ? RUN : run);
     const size_t cs = (size_t)nx * ny;
     const int tid = threadIdx.x;
     const long long nunits = L.ntx * L.nseg;
@@ -448,16 +450,27 @@ int launch_ip(void *f, int nx, int ny, int boundary, double u0, void *ws, size_t
         return LBGB_EINVAL;
     }
     const bool vec = (ny % G::VW == 0) && aligned(f, 16);
-    const int run = vec ? IP_RUN : 1;
+    // The pipelined kernel's blocks take whole runs.  Shorter ones where that
+    // leaves the last block more than a tenth fewer tiles to do (they cost about 3 %
+    // in column records): small lattices have few runs (us with the save: 512^2 as
+    // 128 runs of one tile 6.9, as 32 of four 15.1; 300x200 7.3 and 9.8; 2048^2
+    // 60.6 and 64.5; 4096x2048, 27 tiles in turn instead of 28, 121.5 and 118.7).
+    int run = vec ? IP_RUN : 1;
+    const auto tiles_in_turn = [&](int r) {
+        const long long units = L.ntx * ((L.nty + r - 1) / r);
+        return (units + ip_sm_count() - 1) / ip_sm_count() * (r < L.nty ? r : L.nty);
+    };
+    for (int r = run / 2; r >= 1; r /= 2)
+        if (10 * tiles_in_turn(r) < 9 * tiles_in_turn(run)) run = r;
     const IpLayout LR = ip_layout<raw>(nx, ny, run);
     raw *fp = static_cast<raw *>(f);
     k_ip_save<raw><<<(unsigned)(6 * (LR.ntx + LR.nseg)), IP_THREADS, 0, s>>>(fp, static_cast<raw *>(ws), nx, ny, run);
     int rc = check_launch("k_ip_save");
     if (rc) return rc;
-    // variants: periodic / cavity x generic / pipelined
-    static std::atomic<bool> attr_set[MAX_DEVICES][4];
+    // variants: periodic / cavity x generic / pipelined (runs of IP_RUN / shorter)
+    static std::atomic<bool> attr_set[MAX_DEVICES][6];
     const int dev = current_device();
-    const int variant = (boundary == LBGB_PERIODIC ? 0 : 1) + (vec ? 2 : 0);
+    const int variant = (boundary == LBGB_PERIODIC ? 0 : 1) + (vec ? (run == IP_RUN ? 2 : 4) : 0);
     const size_t smem = vec ? 2 * G::SMEM : G::SMEM;
     auto go = [&](auto kernel, unsigned grid, int threads, const char *name) -> int {
         if (!attr_set[dev][variant].load(std::memory_order_acquire)) {
@@ -469,15 +482,18 @@ int launch_ip(void *f, int nx, int ny, int boundary, double u0, void *ws, size_t
             }
             attr_set[dev][variant].store(true, std::memory_order_release);
         }
-        kernel<<<grid, threads, smem, s>>>(fp, static_cast<const raw *>(ws), nx, ny, (typename Codec<DT>::real)u0);
+        kernel<<<grid, threads, smem, s>>>(fp, static_cast<const raw *>(ws), nx, ny, run, (typename Codec<DT>::real)u0);
         return check_launch(name);
     };
     if (vec) {
         const long long units = LR.ntx * LR.nseg;
         const unsigned grid = (unsigned)(units < ip_sm_count() ? units : ip_sm_count());
-        return boundary == LBGB_PERIODIC
-                   ? go(k_ip_stream_pipe<DT, LBGB_PERIODIC>, grid, IPP_THREADS, "k_ip_stream_pipe")
-                   : go(k_ip_stream_pipe<DT, LBGB_CAVITY>, grid, IPP_THREADS, "k_ip_stream_pipe");
+        const char *name = "k_ip_stream_pipe";
+        if (boundary == LBGB_PERIODIC)
+            return run == IP_RUN ? go(k_ip_stream_pipe<DT, LBGB_PERIODIC, IP_RUN>, grid, IPP_THREADS, name)
+                                 : go(k_ip_stream_pipe<DT, LBGB_PERIODIC, 0>, grid, IPP_THREADS, name);
+        return run == IP_RUN ? go(k_ip_stream_pipe<DT, LBGB_CAVITY, IP_RUN>, grid, IPP_THREADS, name)
+                             : go(k_ip_stream_pipe<DT, LBGB_CAVITY, 0>, grid, IPP_THREADS, name);
     }
     return boundary == LBGB_PERIODIC ? go(k_ip_stream<DT, LBGB_PERIODIC>, (unsigned)tiles, IP_THREADS, "k_ip_stream")
                                      : go(k_ip_stream<DT, LBGB_CAVITY>, (unsigned)tiles, IP_THREADS, "k_ip_stream");
