@@ -17,6 +17,8 @@ for bit.  A time loop that owns its buffers should use
 cell and step).
 """
 
+import functools
+
 import numpy as np
 import torch
 
@@ -30,11 +32,16 @@ c_ic = np.array([[0, 1, 0, -1, 0, 1, -1, -1, 1],
                  [0, 0, 1, 0, -1, 1, 1, -1, -1]]).T
 
 
+@functools.lru_cache(maxsize=64)
+def _workspace_bytes(nx, ny, code):
+    return int(_lib.load().lbgb_stream_inplace_workspace_bytes(nx, ny, code))
+
+
 def _workspace(f_ikl, nx, ny, code):
     """Edge-record workspace of one in-place stream, from torch's caching
     allocator on the tensor's device (stream-ordered: reused only after the
     call that held it)."""
-    nbytes = int(_lib.load().lbgb_stream_inplace_workspace_bytes(nx, ny, code))
+    nbytes = _workspace_bytes(nx, ny, code)
     return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=f_ikl.device), nbytes
 
 

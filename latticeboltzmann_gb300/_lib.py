@@ -158,7 +158,9 @@ def check(rc, what=""):
 
 
 def call(name, *args):
-    check(getattr(load(), name)(*args), name)
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != OK:
+        check(rc, name)
 
 
 def set_tuning(key, value):

@@ -30,8 +30,16 @@ def storage_code(t, name):
         raise TypeError("%s: dtype %s not supported (float32 or float64)" % (name, t.dtype)) from None
 
 
+def stream_of(device):
+    """Handle of the device's current stream: ``torch.cuda.current_stream(device)
+    .cuda_stream`` without the stream object, whose making takes a fifth of a
+    small operator's host time."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
 def stream_handle(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def population_view(f, name):

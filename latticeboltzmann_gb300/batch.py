@@ -19,6 +19,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from ._tensor import stream_of
 from .solver import _RAW, capture_steps, viscosity_from_omega
 
 INSTANCE_DTYPE = np.dtype([("offset", "<i8"), ("nx", "<i4"), ("ny", "<i4"), ("omega", "<f8"), ("u0", "<f8"),
@@ -134,7 +135,7 @@ class BatchedLattice:
         return self._buf[self._cur]
 
     def _stream(self):
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return stream_of(self.device)
 
     def _slice(self, b, buf=None):
         buf = self.state if buf is None else buf
@@ -260,6 +261,21 @@ class BatchedLattice:
             self._step_plans[key] = self._plan()[:2]
         return self._step_plans[key]
 
+    def _schedule(self, n):
+        """(kind, the steps of each launch of several, single steps after them) of ``step(n)``."""
+        kind, most = self._several()
+        several, left = [], n
+        while left > 0 and kind != _lib.BATCH_SINGLE:
+            if kind == _lib.BATCH_TILE:
+                t = -(-left // -(-left // most))
+            else:
+                t = 4 if left >= 4 else 2
+                if left < t:
+                    break
+            several.append(t)
+            left -= t
+        return kind, several, left
+
     def _launch_steps(self, kind, t):
         """One launch of t steps of the active instances."""
         full = self._step_tasks.get((t, None))
@@ -284,20 +300,11 @@ class BatchedLattice:
         """Advance the active instances n steps: several per launch (see
         lbgb_batch_plan; the same results bit for bit), or one per launch of
         ``config`` where one is given or several do not apply."""
-        left = int(n)
-        if config is None:
-            kind, most = self._several()
-            while left > 0 and kind != _lib.BATCH_SINGLE:
-                if kind == _lib.BATCH_TILE:
-                    t = -(-left // -(-left // most))
-                else:
-                    t = 4 if left >= 4 else 2
-                    if left < t:
-                        break
-                self._launch_steps(kind, t)
-                left -= t
+        kind, several, singles = self._schedule(int(n)) if config is None else (None, [], int(n))
+        for t in several:
+            self._launch_steps(kind, t)
         cfg = config or self.config
-        for _ in range(left):
+        for _ in range(singles):
             self._launch(self._buf[self._cur], self._buf[1 - self._cur], cfg)
             self._cur = 1 - self._cur
         self.steps_taken += int(n)

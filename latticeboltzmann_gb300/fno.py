@@ -38,6 +38,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from ._tensor import stream_of
 
 # GEMM engines: tensor cores (the TMA pipeline where both operands are
 # K-major, else the staged kernel), CUDA cores, the staged tensor-core kernel
@@ -158,7 +159,7 @@ class FNO2d:
         _lib.call("lbgb_fno_to_bf16", self.flat.data_ptr(), self.flat_bf16.data_ptr(), self.numel, self._s())
 
     def _s(self):
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return stream_of(self.device)
 
     def state_dict(self):
         return {"config": dict(width=self.width, modes=self.modes, layers=self.layers, hidden=self.hidden,

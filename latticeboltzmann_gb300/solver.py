@@ -16,7 +16,7 @@ import ctypes
 import torch
 
 from . import _lib
-from ._tensor import require_cuda
+from ._tensor import require_cuda, stream_of
 
 _RAW = {"f32": torch.float32, "f64": torch.float64, "f16dev": torch.int16, "bf16dev": torch.int16,
         "f32dev": torch.float32}
@@ -160,7 +160,7 @@ class Lattice:
         return self._buf[self._cur]
 
     def _stream(self):
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return stream_of(self.device)
 
     def load(self, f):
         """Set the populations from a float tensor ``(9, nx, ny)`` on any device.
