@@ -82,7 +82,7 @@ def parse(argv=None):
                    help="rounding of 16-bit storage")
     p.add_argument("--workload", choices=["cavity", "batched-shear"], default="cavity",
                    help="cavity: one lattice (default); batched-shear: 512 uneven periodic shear-wave lattices "
-                        "advanced by one launch per step (autotuned)")
+                        "advanced together, several steps per launch")
     p.add_argument("--no-extras", action="store_true",
                    help="skip the 16-bit storage comparison, the operator-path timing and the warm-start study")
     p.add_argument("--extras", default="operator_path,fp16_store,warm_start",
@@ -749,8 +749,9 @@ def run_batched(args):
     bl = B.BatchedLattice(sizes, om, boundary="periodic", storage=args.storage, device=dev).shear_wave(0.05)
     best, timings = bl.autotune()
     stream = torch.cuda.current_stream(dev)
-    for _ in range(args.warmup):
-        bl.step(1)
+    _, several, singles = bl._schedule(args.steps)
+    for t in [1] * args.warmup + several[:1] + several[-1:]:  # the task lists of the timed launches, too
+        bl.step(t)
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
     d.barrier()
     torch.cuda.synchronize(dev)
@@ -764,20 +765,22 @@ def run_batched(args):
     mlups, t_max = aggregate_mlups(bl.cells, args.steps, secs, d, dev)
     if d.rank == 0:
         bpc = 18 * torch.empty(0, dtype=bl.state.dtype).element_size()
-        achieved = bpc * bl.cells / (secs / args.steps) / 1e9
+        launches = len(several) + singles
+        achieved = bpc * bl.cells * launches / secs / 1e9
         peak, peak_src = hbm_peak()
         print(json.dumps({
-            "metric": "MLUPS (512 batched uneven D2Q9 shear-wave lattices, one launch per step)",
+            "metric": "MLUPS (512 batched uneven D2Q9 shear-wave lattices)",
             "value": round(mlups, 1), "unit": UNIT, "n_gpus": d.world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": round(t_max / args.steps * 1e3, 4), "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64" if args.storage == "f64" else "f32", "data": "synthetic (seeded batch)",
             "config": {"workload": "512 periodic shear-wave lattices, nx log-uniform 32..1024, ny 16..512, "
                                    "omega 0.3..1.9, seed 0, %s" % args.storage, "cells": bl.cells,
                        "launch": bl.config},
-            "gpu_launches": args.steps,
+            "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": None, "peak_source": peak_src,
-                         "kernel": "k_batch_step_flat / k_batch_step (autotuned)"},
+                         "kernel": "k_march_batch (several steps per launch) / k_batch_step_flat / k_batch_step (autotuned)",
+                         "steps_per_launch": round(args.steps / launches, 2)},
         }), flush=True)
     d.close()
     return 0

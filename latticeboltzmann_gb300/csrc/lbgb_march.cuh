@@ -28,7 +28,7 @@
 // through shared-memory tiles 89,800 (97 % of the copy bandwidth); two steps
 // per launch in 128-column blocks with block barriers and scalar FP32 128,100;
 // this kernel T = 2 155,000, T = 3 226,000, T = 4 252,000 (periodic 268,000;
-// f32dev 290,000; half 283,000 and bfloat16 303,000 against 169,000 and
+// f32dev 298,000; half 283,000 and bfloat16 303,000 against 169,000 and
 // 171,000 with one step per launch).  A second input row in flight measured
 // slower (T = 3 periodic 222,000 against 238,000), 16 warps of 128 registers
 // too (205,000).  The wall rules run in separate instances of the row
