@@ -450,17 +450,19 @@ int launch_ip(void *f, int nx, int ny, int boundary, double u0, void *ws, size_t
         return LBGB_EINVAL;
     }
     const bool vec = (ny % G::VW == 0) && aligned(f, 16);
-    // The pipelined kernel's blocks take whole runs.  Shorter ones where that
-    // leaves the last block more than a tenth fewer tiles to do (they cost about 3 %
-    // in column records): small lattices have few runs (us with the save: 512^2 as
-    // 128 runs of one tile 6.9, as 32 of four 15.1; 300x200 7.3 and 9.8; 2048^2
-    // 60.6 and 64.5; 4096x2048, 27 tiles in turn instead of 28, 121.5 and 118.7).
+    // The pipelined kernel's blocks take whole runs.  Shorter ones where a block
+    // has up to four runs to do and that leaves it more than a tenth fewer tiles
+    // (they cost about 3 % in column records): small lattices have few runs (us with
+    // the save: 512^2 as 128 runs of one tile 6.9, as 32 of four 15.1; 300x200 7.3
+    // and 9.8; 2048^2 60.6 and 64.5).  With more runs a block the early ones leave
+    // their bandwidth to the rest (2212x3704, 28 tiles in turn instead of 32: 1.5 %
+    // slower with the walls' collision; 4096x2048, 27 of 28: 121.5 and 118.7).
     int run = vec ? IP_RUN : 1;
     const auto tiles_in_turn = [&](int r) {
         const long long units = L.ntx * ((L.nty + r - 1) / r);
         return (units + ip_sm_count() - 1) / ip_sm_count() * (r < L.nty ? r : L.nty);
     };
-    for (int r = run / 2; r >= 1; r /= 2)
+    for (int r = run / 2; r >= 1 && tiles_in_turn(IP_RUN) <= 4 * IP_RUN; r /= 2)
         if (10 * tiles_in_turn(r) < 9 * tiles_in_turn(run)) run = r;
     const IpLayout LR = ip_layout<raw>(nx, ny, run);
     raw *fp = static_cast<raw *>(f);
