@@ -20,7 +20,7 @@ import torch
 
 from . import _lib
 from ._tensor import stream_of
-from .solver import _RAW, capture_steps, viscosity_from_omega
+from .solver import _RAW, Replay, viscosity_from_omega
 
 INSTANCE_DTYPE = np.dtype([("offset", "<i8"), ("nx", "<i4"), ("ny", "<i4"), ("omega", "<f8"), ("u0", "<f8"),
                            ("vec", "<i4"), ("cell_base", "<u4")])
@@ -311,7 +311,9 @@ class BatchedLattice:
         return self
 
     def capture(self, n):
-        """CUDA graph of ``n`` (even) steps; returns a callable replaying them."""
+        """CUDA graphs of ``n`` (even) steps of the instances active now; returns a
+        callable that advances the batch by them (see ``Replay``).  It may be
+        mixed with ``step``; read ``state`` after a replay."""
         if n <= 0 or n % 2:
             raise ValueError("capture: n must be a positive even number")
         self.task_queue(self.config["vector"], self.config["rows"], self.config.get("flat", False))  # outside the capture
@@ -323,7 +325,7 @@ class BatchedLattice:
         self._buf[cur].copy_(saved)
         self._cur, self.steps_taken = cur, taken
         torch.cuda.synchronize(self.device)
-        return capture_steps(self, n)
+        return Replay(self, n)
 
     # ------------------------------------------------------------ diagnostics
     def shear_amplitudes(self, out=None):

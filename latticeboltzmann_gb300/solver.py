@@ -38,38 +38,61 @@ def viscosity_from_omega(omega):
     return (1.0 / omega - 0.5) / 3.0
 
 
-def capture_steps(lattice, n):
-    """CUDA graph of ``lattice.step(n)``; returns a callable replaying it.
+class Replay:
+    """Advances ``lattice`` (a ``Lattice`` or a ``BatchedLattice``) n steps per
+    call by a CUDA graph of ``lattice.step(n)``.
 
-    A graph holds the addresses of the two buffers.  Where the launches of n
-    steps (several steps each) are odd in number, the state ends in the other
-    buffer: a second graph starts from there, and the replays alternate."""
-    graphs = {}
-    start = lattice._cur
-    for cur in (start, 1 - start):
-        lattice._cur = cur
+    A graph holds the addresses of the two buffers, and the state may be in
+    either when a replay begins: n steps, several per launch, may be an odd
+    number of launches, and so may the steps that the caller takes between
+    replays.  So there is one graph per buffer, and a call replays the one that
+    starts where the state is.  The state may then be in the other buffer: read
+    ``lattice.state`` again after a replay, as after ``step``.
+    """
+
+    def __init__(self, lattice, n):
+        self._lattice, self._n = lattice, n
+        self._closed = {}
+        self._graphs = {cur: self._record(cur, (n,)) for cur in (lattice._cur, 1 - lattice._cur)}
+
+    def _record(self, cur, parts):
+        """(graph of ``step(k) for k in parts`` from buffer ``cur``, the buffer it ends in)."""
+        lattice = self._lattice
+        saved, taken = lattice._cur, lattice.steps_taken
         s = torch.cuda.Stream(device=lattice.device)
         s.wait_stream(torch.cuda.current_stream(lattice.device))
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s):
-            with torch.cuda.graph(g, stream=s):
-                lattice.step(n)
+        try:
+            lattice._cur = cur
+            with torch.cuda.stream(s):
+                with torch.cuda.graph(g, stream=s):
+                    for k in parts:
+                        lattice.step(k)
+            end = lattice._cur
+        finally:
+            # launches were recorded, none has run
+            lattice._cur, lattice.steps_taken = saved, taken
         torch.cuda.current_stream(lattice.device).wait_stream(s)
-        lattice.steps_taken -= n
-        graphs[cur] = (g, lattice._cur)
-        if lattice._cur == cur:
-            break
-    lattice._cur = start
+        return g, end
 
-    def replay():
-        g, end = graphs.get(lattice._cur) or graphs[start]
+    def __call__(self):
+        lattice = self._lattice
+        g, end = self._graphs[lattice._cur]
         g.replay()
-        if len(graphs) == 2:
-            lattice._cur = end
-        lattice.steps_taken += n
+        lattice._cur = end
+        lattice.steps_taken += self._n
 
-    replay.graph = graphs[start][0]
-    return replay
+    @property
+    def graph(self):
+        """A graph of the n steps that ends in the buffer it starts from, the one
+        that holds the state when this is read (two halves take equally many
+        launches).  Replaying it oneself leaves ``steps_taken`` as it is."""
+        cur = self._lattice._cur
+        if self._graphs[cur][1] == cur:
+            return self._graphs[cur][0]
+        if cur not in self._closed:
+            self._closed[cur] = self._record(cur, (self._n // 2, self._n // 2))[0]
+        return self._closed[cur]
 
 
 class Lattice:
@@ -368,10 +391,9 @@ class Lattice:
         return self
 
     def capture(self, n):
-        """Capture ``n`` steps into a CUDA graph; returns a callable replaying them.
-
-        ``n`` must be even.
-        """
+        """Capture ``n`` (even) steps into CUDA graphs; returns a callable that
+        advances the lattice by them (see ``Replay``).  It may be mixed with
+        ``step`` and with loading a state; read ``state`` after a replay."""
         if n <= 0 or n % 2:
             raise ValueError("capture: n must be a positive even number")
         # load the kernel variant outside the capture: one step on a two-row
@@ -385,7 +407,7 @@ class Lattice:
                       self.omega, self.u0, self.code, 1, self.seed, ctr.data_ptr(), ctypes.byref(ctypes.c_int(0)),
                       self._stream())
         torch.cuda.current_stream(self.device).synchronize()
-        return capture_steps(self, n)
+        return Replay(self, n)
 
     # ------------------------------------------------------------------ diagnostics
     def macroscopic(self):

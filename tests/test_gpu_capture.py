@@ -1,0 +1,69 @@
+"""Captured steps mixed with ordinary ones against single steps, bit for bit:
+lattices and batches whose steps take even and odd numbers of launches."""
+
+import numpy as np
+import pytest
+import torch
+
+import latticeboltzmann_gb300 as PyLB
+from latticeboltzmann_gb300 import _lib
+from latticeboltzmann_gb300 import batch as B
+from test_gpu_batch_steps import LARGE, SINGLE, SMALL, make
+from test_gpu_march import two_step  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def mixed(lat, n, m):
+    replay = lat.capture(n)
+    for part in (n, m, n, n, m, n):
+        replay() if part == n else lat.step(part)
+    return replay, 4 * n + 2 * m
+
+
+@pytest.mark.parametrize("size,storage,rounding", [((256, 256), "f32", "nearest"), ((1237, 1288), "f32", "nearest"),
+                                                   ((256, 256), "f16dev", "stochastic"), ((96, 80), "f64", "nearest")])
+@pytest.mark.parametrize("n", [8, 10])
+@pytest.mark.parametrize("m", [2, 3, 4])
+def test_lattice_replays_mixed_with_steps(two_step, cuda, size, storage, rounding, n, m):
+    def lattice():
+        lat = PyLB.Lattice(*size, 1.4, boundary="cavity", u0=0.05, storage=storage, rounding=rounding, seed=5, device=cuda)
+        return lat.equilibrium(1.0, 0.01, 0.02)
+    _lib.set_tuning(_lib.TUNE_TWO_STEP, 1)
+    lat, ref = lattice(), lattice()
+    replay, total = mixed(lat, n, m)
+    _lib.set_tuning(_lib.TUNE_TWO_STEP, 0)
+    for _ in range(total):
+        ref.step(1)
+    assert lat.steps_taken == total
+    assert torch.equal(lat.state, ref.state)
+    # the graph itself keeps the buffer
+    replay.graph.replay()
+    for _ in range(n):
+        ref.step(1)
+    assert torch.equal(lat.state, ref.state)
+
+
+@pytest.mark.parametrize("sizes", [SMALL, LARGE])
+@pytest.mark.parametrize("n", [8, 10])
+@pytest.mark.parametrize("m", [2, 3, 4])
+def test_batch_replays_mixed_with_steps(cuda, sizes, n, m):
+    a, b = make(sizes, "f32", "periodic", cuda), make(sizes, "f32", "periodic", cuda)
+    _, total = mixed(a, n, m)
+    b.step(total, SINGLE)
+    assert a.steps_taken == total
+    assert torch.equal(a.state, b.state)
+
+
+def test_state_loaded_between_replays(two_step, cuda):
+    _lib.set_tuning(_lib.TUNE_TWO_STEP, 1)
+    lat = PyLB.Lattice(256, 256, 1.4, u0=0.05, device=cuda)
+    ref = PyLB.Lattice(256, 256, 1.4, u0=0.05, device=cuda)
+    replay = lat.capture(2)  # one launch
+    replay()
+    f = ref.equilibrium(1.01, 0.0, 0.01).populations()
+    lat.load(f)
+    ref.load(f)
+    replay()
+    ref.step(2)
+    assert torch.equal(lat.state, ref.state)
