@@ -16,10 +16,10 @@
 // dereferenced.
 #pragma once
 
-#include <algorithm>
-#include <vector>
+#include <exception>
 
 #include "lbgb_batch.h"
+#include "lbgb_batch_plan.h"
 
 namespace lbgb {
 
@@ -445,82 +445,6 @@ extern "C" int lbgb_batch_velocity_change(const void *f, long long total_elems, 
     return check_launch("k_batch_change_finish");
 }
 
-namespace lbgb {
-
-// Lanes that write a strip of `left` columns at the lowest cost, and the lanes
-// of the strip itself: 32, 16 or 8, two of which only feed their neighbours.
-static int batch_lanes(int left, int *first) {
-    static const int kinds[] = {32, 16, 8};
-    if (left <= 0) return 0;
-    if (left > 4096) {
-        *first = 32;
-        return 32 + batch_lanes(left - 120, first);
-    }
-    thread_local std::vector<int> cost, kind;
-    if (cost.empty()) cost.push_back(0), kind.push_back(0);
-    for (int c = (int)cost.size(); c <= left; ++c) {
-        int best = 0, k = 0;
-        for (int g : kinds) {
-            const int rest = c - 4 * (g - 2), n = g + (rest > 0 ? cost[rest] : 0);
-            if (!k || n < best) best = n, k = g;
-        }
-        cost.push_back(best);
-        kind.push_back(k);
-    }
-    *first = kind[left];
-    return cost[left];
-}
-
-struct BatchTask {
-    int x, y, z, w;
-};
-
-// March: chunks of `target` rows of every strip.
-static void batch_march_tasks(const int *nx, const int *ny, int n, bool walls, int T, int target,
-                              std::vector<BatchTask> &out) {
-    out.clear();
-    for (int b = 0; b < n; ++b) {
-        const int most = std::max(1, std::min(target, nx[b] - T));
-        for (int y = 0; y < ny[b];) {
-            int g = 32;
-            if (!walls) batch_lanes(ny[b] - y, &g);
-            const int groups = 32 / g;
-            int chunks = (nx[b] + most - 1) / most;
-            chunks = (chunks + groups - 1) / groups * groups;
-            int rows = (nx[b] + chunks - 1) / chunks;
-            for (int x = 0; x < nx[b]; x += rows * groups) out.push_back({b, x, y, rows | (g << 16)});
-            y += 4 * (g - 2);
-        }
-    }
-}
-
-// Tiles of T steps; each instance's shape for its share of the SMs.  Returns
-// the expected cycles per step, or 0 where an instance has no tile.
-static double batch_tile_tasks(const int *nx, const int *ny, int n, int T, int element, double cell, int sms,
-                               std::vector<BatchTask> &out) {
-    out.clear();
-    double all = 0.0, work = 0.0;
-    for (int b = 0; b < n; ++b) all += (double)nx[b] * ny[b];
-    for (int b = 0; b < n; ++b) {
-        const double share = sms * ((double)nx[b] * ny[b] / all);
-        const int m = share < 1.0 ? 1 : (int)(share + 0.5);
-        if (T > nx[b] || T > ny[b]) return 0.0;
-        const TileShape t = tile_shape(nx[b], ny[b], T, element, cell, m);
-        if (!t.rows || t.rows > 0xffff) return 0.0;
-        const int co = std::min(t.cols, ny[b]);
-        for (int x = 0; x < nx[b]; x += t.rows)
-            for (int y = 0; y < ny[b]; y += co) {
-                const int ro = std::min(t.rows, nx[b] - x), c = std::min(co, ny[b] - y);
-                out.push_back({b, x, y, ro | (c << 16)});
-            }
-        // one instance on m SMs
-        work += tile_cost(nx[b], ny[b], t, cell, m) * T * m;
-    }
-    return work / sms / T;
-}
-
-}  // namespace lbgb
-
 extern "C" int lbgb_batch_plan(const int *nx, const int *ny, int n, int boundary, int dtype, int steps, int *kind,
                                int *most, int *tasks, long long capacity, long long *n_tasks) {
     using namespace lbgb;
@@ -536,68 +460,30 @@ extern "C" int lbgb_batch_plan(const int *nx, const int *ny, int n, int boundary
         set_error("lbgb_batch_plan: unknown boundary code %d", boundary);
         return LBGB_EINVAL;
     }
-    const int es = (int)raw_size(dtype), sms = sm_count();
-    const bool walls = boundary != LBGB_PERIODIC;
-    double cells = 0.0;
-    bool march = es == 4, tile = true;
-    for (int b = 0; b < n; ++b) {
+    for (int b = 0; b < n; ++b)
         if (nx[b] <= 0 || ny[b] <= 0) {
             set_error("lbgb_batch_plan: instance %d has size %d x %d", b, nx[b], ny[b]);
             return LBGB_EINVAL;
         }
-        cells += (double)nx[b] * ny[b];
-        march = march && nx[b] >= 8 && ny[b] >= 16;
-        tile = tile && nx[b] >= 2 && ny[b] >= 2 && ny[b] <= 0x7fff;
-    }
     *kind = LBGB_BATCH_SINGLE;
     *most = 1;
     *n_tasks = 0;
     if (!g_tune.two_step) return LBGB_OK;
-    std::vector<BatchTask> list;
-    // the march for large batches of 4-byte codes, tiles for small ones
-    const double tile_most = dtype == LBGB_F64 ? 150000 : 1200000;
-    if (march && cells > tile_most) {
-        *kind = LBGB_BATCH_MARCH;
-        *most = 4;
-        const int T = steps == 2 ? 2 : 4;
-        // rows of a chunk: as march_chunks, over the warps of the whole batch
-        static const int targets[] = {4, 8, 12, 16, 24, 32, 48, 64, 96, 128};
-        double least = 0.0;
-        int best = 4;
-        for (int r : targets) {
-            double warps = 0.0;
-            batch_march_tasks(nx, ny, n, walls, T, r, list);
-            warps = (double)list.size();
-            const double load = warps / (4.0 * sms), cost = (r + 2 * T - 1) * ((load > 1.9 ? load : 1.9) + 1.0);
-            if (least == 0.0 || cost < least) least = cost, best = r;
-        }
-        batch_march_tasks(nx, ny, n, walls, T, best, list);
-        // the longest chunks first
-        std::stable_sort(list.begin(), list.end(),
-                         [](const BatchTask &a, const BatchTask &c) { return (a.w & 0xffff) > (c.w & 0xffff); });
-    } else if (tile && cells <= tile_most) {
-        const double cell = dtype == LBGB_F64 ? 13.5 : 1.45;
-        double least = 0.0;
-        int best = 0;
-        for (int T = 2; T <= TILE_MAX_STEPS; ++T) {
-            const double c = batch_tile_tasks(nx, ny, n, T, es, cell, sms, list);
-            if (c > 0.0 && (!best || c < least)) least = c, best = T;
-        }
-        if (best < 2) return LBGB_OK;
-        *kind = LBGB_BATCH_TILE;
-        *most = best;
-        const int T = steps >= 1 && steps < best ? steps : best;
-        if (batch_tile_tasks(nx, ny, n, T, es, cell, sms, list) == 0.0) return LBGB_OK;
-    } else {
-        return LBGB_OK;
+    BatchForm f;
+    try {
+        f = batch_form(nx, ny, n, boundary, dtype, (int)raw_size(dtype), steps, sm_count(),
+                       BatchSink{reinterpret_cast<BatchTask *>(tasks), capacity});
+    } catch (const std::exception &e) {
+        set_error("lbgb_batch_plan: %s", e.what());
+        return LBGB_EINVAL;
     }
-    if (list.size() > 0x7fffffffull) {
+    if (f.n_tasks > 0x7fffffffll) {
         set_error("lbgb_batch_plan: too many tasks");
         return LBGB_EINVAL;
     }
-    *n_tasks = (long long)list.size();
-    const long long m = std::min<long long>(capacity, *n_tasks);
-    if (m > 0) memcpy(tasks, list.data(), (size_t)m * sizeof(BatchTask));
+    *kind = f.kind;
+    *most = f.most;
+    *n_tasks = f.n_tasks;
     return LBGB_OK;
 }
 
