@@ -85,10 +85,11 @@ inline int chunk_rows(int nx, int T, int target, int g, long long *tasks) {
 
 constexpr int MARCH_MOST_ROWS = 128;
 
-// Tasks by the rows of their chunks.
+// Tasks by the rows of their chunks, and those of instances without whole
+// 16-byte vectors.
 struct MarchCount {
     long long of_rows[MARCH_MOST_ROWS + 1] = {};
-    long long total = 0;
+    long long total = 0, ragged = 0;
 };
 
 inline void march_count(const int *nx, const int *ny, int n, bool walls, int T, int target,
@@ -104,6 +105,7 @@ inline void march_count(const int *nx, const int *ny, int n, bool walls, int T, 
             const int rows = chunk_rows(nx[b], T, target, lanes[k], &tasks);
             c.of_rows[rows] += tasks * it->second[k];
             c.total += tasks * it->second[k];
+            if (ny[b] % 4) c.ragged += tasks * it->second[k];
         }
     }
 }
@@ -159,7 +161,37 @@ inline double tile_tasks(const int *nx, const int *ny, int n, int T, int element
 }
 
 // ---------------------------------------------------------------- plan
-// The march for large batches of 4-byte codes, tiles for small ones.
+// Expected SM cycles per step of one step per launch: 6700 for the launch and
+// 0.0246 a cell (periodic) or 0.031 (walls) over 152 SMs, FP64 0.071 and 0.096
+// (measured: 78,000 and 62,000 MLUPS FP32, 27,000 and 20,000 FP64).
+inline double batch_single_cost(double cells, bool walls, int dtype, int sms) {
+    const double cell = dtype == LBGB_F64 ? (walls ? 0.096 : 0.071) : (walls ? 0.031 : 0.0246);
+    return 6700 + cells * cell * (152.0 / sms);
+}
+
+// And of a march of four: an iteration of a warp takes 1790 cycles (periodic),
+// 3360 (cavity) or 2590 (wall-density-1 lid), with rows of whole vectors; without
+// them 2590, 3940, 3110; f32dev 0.93 of that (periodic) or 0.84.  (The wall rules
+// run in a row of their own kind, and a narrow instance has no strip without them.)
+inline double batch_march_cost(const MarchCount &c, int boundary, int dtype, int sms) {
+    static const double vec[] = {1790, 3360, 2590}, odd[] = {2590, 3940, 3110};
+    const double load = (double)c.total / (4.0 * sms), part = (double)c.ragged / (double)c.total;
+    double rows = 0.0;
+    for (int r = 1; r <= MARCH_MOST_ROWS; ++r) rows += (double)r * c.of_rows[r];
+    const double iteration = (vec[boundary] * (1.0 - part) + odd[boundary] * part) *
+                             (dtype == LBGB_F32 ? 1.0 : (boundary == LBGB_PERIODIC ? 0.93 : 0.84));
+    return iteration * (rows / c.total + 6.0) * ((load > 1.9 ? load : 1.9) + 1.0) / 4.0;
+}
+
+// The march for large batches of 4-byte codes, tiles for small ones, unless one
+// step per launch is expected to be faster: narrow instances fill few of a warp's
+// lanes, short ones are mostly halo, and a tile's fixed cost is that of a few
+// thousand cells.  us a step of FP32 cavities, several steps and one per launch:
+// 8000 of 16^2 174 and 43, 3000 of 32^2 116 and 60, 700 of 65^2 84 and 54, 2400 of
+// 64^2 176 and 170, 152 of 256^2 125 and 144; 68750 of 4^2 467 and 41, 4300 of 16^2
+// 28 and 22, 1100 of 32^2 14 and 22.  Over 455 batches of 1.3 to 10 M cells and
+// 507 of 10 k to 1.1 M the costs take the slower form in 6 %, by 9 % in the
+// median; the factors lean to several steps, which also take fewer calls.
 inline double batch_tile_most(int dtype) { return dtype == LBGB_F64 ? 150000 : 1200000; }
 
 struct BatchForm {
@@ -181,19 +213,25 @@ inline BatchForm batch_form(const int *nx, const int *ny, int n, int boundary, i
     }
     BatchForm f;
     if (march && cells > batch_tile_most(dtype)) {
-        const int T = steps == 2 ? 2 : 4;
         // rows of a chunk: as march_chunks, over the warps of the whole batch
         static const int targets[] = {4, 8, 12, 16, 24, 32, 48, 64, 96, MARCH_MOST_ROWS};
         std::unordered_map<int, std::array<long long, 3>> strips;
         MarchCount count, best;
-        double least = 0.0;
         int target = 0;
-        for (int r : targets) {
-            march_count(nx, ny, n, walls, T, r, strips, count);
-            const double load = (double)count.total / (4.0 * sms),
-                         cost = (r + 2 * T - 1) * ((load > 1.9 ? load : 1.9) + 1.0);
-            if (!target || cost < least) least = cost, target = r, best = count;
-        }
+        auto cut = [&](int T) {
+            double least = 0.0;
+            target = 0;
+            for (int r : targets) {
+                march_count(nx, ny, n, walls, T, r, strips, count);
+                const double load = (double)count.total / (4.0 * sms),
+                             cost = (r + 2 * T - 1) * ((load > 1.9 ? load : 1.9) + 1.0);
+                if (!target || cost < least) least = cost, target = r, best = count;
+            }
+        };
+        cut(4);
+        if (batch_march_cost(best, boundary, dtype, sms) > 1.05 * batch_single_cost(cells, walls, dtype, sms)) return f;
+        const int T = steps == 2 ? 2 : 4;
+        if (T == 2) cut(2);
         f.kind = LBGB_BATCH_MARCH;
         f.most = 4;
         f.n_tasks = best.total;
@@ -208,7 +246,7 @@ inline BatchForm batch_form(const int *nx, const int *ny, int n, int boundary, i
             const double c = tile_tasks(nx, ny, n, T, element, cell, sms, shapes, BatchSink{nullptr, 0}, &count);
             if (c > 0.0 && (!best || c < least)) least = c, best = T;
         }
-        if (best < 2) return f;
+        if (best < 2 || least > 1.1 * batch_single_cost(cells, walls, dtype, sms)) return f;
         f.kind = LBGB_BATCH_TILE;
         f.most = best;
         const int T = steps >= 1 && steps < best ? steps : best;

@@ -336,7 +336,10 @@ static Several several_steps(const void *src, const void *dst, int nx, int ny, i
             tile_plan(p, nx, ny, kind, es, dtype == LBGB_F64 ? 13.5 : (sr ? 4.0 : 1.45), sms);
             m.plan = &p;
         }
-        if (m.plan->steps > 1) {
+        // (stochastic rounding takes 0.55 of the cycles its plans are made with)
+        const bool slower = !m.ragged && dtype != LBGB_F64 &&
+                            m.plan->cost * (sr ? 0.55 : 1.0) > single_cost((double)cells, es, m.plan->sms);
+        if (m.plan->steps > 1 && !slower) {
             m.kind = Several::TILE;
             m.most = m.plan->steps;
             return m;

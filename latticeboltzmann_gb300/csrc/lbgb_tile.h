@@ -84,6 +84,7 @@ inline TileShape tile_shape(int nx, int ny, int T, int element, double cell, int
 // The shapes of every step count for one kind of lattice, and the best count.
 struct TilePlan {
     int nx = 0, ny = 0, kind = -1, sms = 0, steps = 0;
+    double cost = 0.0;  // of the best count
     TileShape shape[TILE_MAX_STEPS + 1];
 };
 inline void tile_plan(TilePlan &p, int nx, int ny, int kind, int element, double cell, int sms) {
@@ -104,6 +105,17 @@ inline void tile_plan(TilePlan &p, int nx, int ny, int kind, int element, double
             p.steps = T;
         }
     }
+    p.cost = least;
+}
+
+// Expected SM cycles of one step in a launch of its own, rows of whole vectors:
+// 5800 for the launch and 0.0205 a cell over 152 SMs (94,000 MLUPS), 16-bit codes
+// 0.0154.  Lattices two to five rows high have tiles that are mostly halo, and
+// one step per launch is faster (2 x 400,000 FP32 12.3 us against 19.3, half 9.9
+// against 15.4; 5 x 200,000 half 10.3 against 13.6).  Rows without whole vectors
+// are slower one step at a time than any tile; FP64 differs by a tenth at most.
+inline double single_cost(double cells, int element, int sms) {
+    return 5800 + cells * (element == 2 ? 0.0154 : 0.0205) * (152.0 / sms);
 }
 
 template <int DT>
