@@ -2,20 +2,24 @@
 //
 // The FP64 units set the time of an FP64 step on this GPU (two operations per
 // SM and clock: ~84 a cell, 7.1 GLUPS; memory would allow 47), while its
-// integer units do 64 operations per SM and clock.  Populations of a flow
-// that BGK can compute lie in (2^-21, 1), so a node's nine values are taken to
-// integers in units of 2^-61 (finer than their own last place from 2^-8 up:
-// the conversion is then exact), summed there without rounding, relaxed with
-// multiplications that keep 64 bits, and rounded once when they are stored.
-// Only 1/rho and the three products j_a j_b / rho use the FP64 units (11
-// operations), whose results enter with the weights 1/2, 1/8 and 1/4.  Mass
-// and momentum change only in the final rounding.  Against 80-bit arithmetic
-// over random states the largest error of a population is smaller than that
-// of the FP64 evaluation (the test states both).
+// integer units do 64 operations per SM and clock.  A node's nine values are
+// taken to integers in units of 2^-61, the last place of doubles from 2^-9 up,
+// so exactly; summed there without rounding, relaxed with multiplications that
+// keep 64 bits, and rounded once when they are stored.  Only 1/rho and the three
+// products j_a j_b / rho use the FP64 units (11 operations), whose results enter
+// with the weights 1/2, 1/8 and 1/4.  Mass and momentum change only in the final
+// rounding.  Against 80-bit arithmetic the largest and the root mean square
+// error of each population are no larger than those of the FP64 evaluation, over
+// the whole range that is taken (the test states both).
 //
-// Nodes outside the range (a population outside (2^-21, 1/2), the rest
-// population outside (2^-21, 1), rho outside [3/4, 3/2), |j| of a component
-// from 0.2 up, NaN, infinity, omega outside [0, 2)) take the FP64 evaluation.
+// Nodes outside the range take the FP64 evaluation: a population outside [2^-9,
+// 1/2), the rest population outside [2^-9, 1), a result outside [2^-9, 1), rho
+// outside [3/4, 3/2), |j| of a component from 0.2 up, NaN, infinity, omega other
+// than 0 outside [1/4, 2).  Below 2^-9 a unit is coarser than a double's last
+// place (a population of 2^-20 would keep 41 bits), and below omega = 0.21 the
+// FP64 evaluation moves the populations so little that the products cut to a
+// unit are the larger error (7 % more root mean square at 0.1).  Populations of
+// a cavity or a wave stay above 2^-6.
 #pragma once
 
 #include <stdint.h>
@@ -49,10 +53,11 @@ inline double fma64(double a, double b, double c) { return __builtin_fma(a, b, c
 #define LBGB_FIX inline
 #endif
 
-// A double in (2^-21, 1) in units of 2^-61 (bits below are dropped: none from
-// 2^-8 up).  `worst` collects the largest shift: values outside give one
+// A double in [2^-21, 1) in units of 2^-61 (bits below are dropped: none from
+// 2^-9 up).  `worst` collects the largest shift: values outside give one
 // beyond MAX_SHIFT (negative numbers, NaN and infinity too).
 constexpr uint32_t MAX_SHIFT = 23;
+constexpr uint32_t EXACT_SHIFT = 11;  // that of [2^-9, 2^-8): nothing is dropped
 LBGB_FIX uint64_t to_fix(double x, uint32_t least, uint32_t &worst) {
     const uint64_t b = bits(x);
     const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
@@ -105,9 +110,11 @@ __host__ __device__ constexpr Factor factor(uint64_t k) {
 constexpr Factor INV3 = factor(0x5555555555555555ull), INV12 = factor(0x1555555555555555ull),
                  INV36 = factor(0x071c71c71c71c71cull);  // 2^64 / 3, / 12, / 36
 
-// omega 2^61; false outside [0, 2)
+// omega 2^61; false unless 0 or in [1/4, 2)
 LBGB_FIX bool omega_factor(double omega, Factor &k) {
-    const bool ok = omega >= 0.0 && omega < 2.0;
+    // by its words: a comparison of doubles takes the FP64 units once a node
+    const uint64_t b = bits(omega);
+    const bool ok = (b << 1) == 0 || (uint32_t)(b >> 32) - 0x3fd00000u < 0x300000u;
     k = factor(ok ? (uint64_t)(long long)(omega * 0x1p61) : 0ull);
     return ok;
 }
@@ -129,11 +136,11 @@ struct Node {
 LBGB_FIX bool load_node(const double (&f)[9], Node &n) {
     uint32_t worst = 0;
     n.x[0] = to_fix(f[0], 3u, worst);
-    bool ok = worst <= MAX_SHIFT - 3u;
+    bool ok = worst <= EXACT_SHIFT - 3u;
     worst = 0;
 #pragma unroll
     for (int i = 1; i < 9; ++i) n.x[i] = to_fix(f[i], 4u, worst);
-    ok = ok && worst <= MAX_SHIFT - 4u;
+    ok = ok && worst <= EXACT_SHIFT - 4u;
     const int64_t a13 = (int64_t)(n.x[1] - n.x[3]), a24 = (int64_t)(n.x[2] - n.x[4]);
     n.a57 = (int64_t)(n.x[5] - n.x[7]);
     n.a68 = (int64_t)(n.x[6] - n.x[8]);
@@ -155,7 +162,7 @@ LBGB_FIX bool in_range(const Node &n) {
            (uint32_t)((uint64_t)n.jy >> 32) + j < 2 * j;
 }
 
-// The moments as doubles, to 2^-52 (rho) and 2^-53 (j): built under a power of
+// The moments as doubles, to 2^-51 (rho) and 2^-53 (j): built under a power of
 // two and freed of it by one subtraction.
 LBGB_FIX double rho_double(uint64_t rho) { return from_bits(0x4000000000000000ull | (rho >> 10)) - 2.0; }
 LBGB_FIX double j_double(int64_t j) {
@@ -190,14 +197,15 @@ LBGB_FIX bool collide(const double (&f)[9], Factor omega, double (&out)[9]) {
                            n.x[6] + (uint64_t)(p68 + o68),
                            n.x[7] + (uint64_t)(p57 - o57),
                            n.x[8] + (uint64_t)(p68 - o68)};
-    // every result in [2^-21, 1): a positive high word with a bit from 2^-21 up
+    // every result in [2^-9, 1): a positive high word with a bit from 2^-9 up
+    constexpr uint32_t LEAST = 0x100000u;
     uint32_t worst = 0;
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
-        const uint32_t e = (uint32_t)(r[i] >> 32) - 0x100u;
+        const uint32_t e = (uint32_t)(r[i] >> 32) - LEAST;
         worst = worst > e ? worst : e;
     }
-    if (worst >= 0x20000000u - 0x100u) return false;
+    if (worst >= 0x20000000u - LEAST) return false;
 #pragma unroll
     for (int i = 0; i < 9; ++i) out[i] = to_double(r[i]);
     return true;
