@@ -119,7 +119,11 @@ LBGB_FIX bool omega_factor(double omega, Factor &k) {
     return ok;
 }
 
-// 1 / x to about 2^-60: the hardware's seed (2^-20) and one cubic step.
+// 1 / x to two last places or so: the hardware's approximation y and one step of
+// the hyperpower iteration of order three, y + y (e + e^2) with e = 1 - x y (M.
+// Altman, Pacific J. Math. 10 (1960) 1107), which leaves e^3 of its error and the
+// roundings of y and of the sum.  The GPU tests compare the collision and the
+// velocities that use it with extended precision.
 LBGB_FIX double rcp(double x) {
     const double y = rcp_seed(x), e = fma64(-x, y, 1.0);
     return fma64(fma64(e, e, e), y, y);
