@@ -108,14 +108,14 @@ class BatchedLattice:
         key = (bool(vector), int(rows), bool(flat), None)
         if key not in self._tasks:
             parts = []
-            for b, (nx, ny) in enumerate(self.sizes):
-                if flat:
-                    c0 = np.arange(0, nx * ny, 32 * rows, dtype=np.int64)
-                    q = np.zeros((c0.size, 4), dtype=np.int32)
-                    q[:, 0] = b
-                    q[:, 2] = c0
-                    parts.append(q)
-                    continue
+            if flat:
+                cells = self._table_np["nx"].astype(np.int64) * self._table_np["ny"]
+                count = -(-cells // (32 * rows))
+                q = np.zeros((int(count.sum()), 4), dtype=np.int32)
+                q[:, 0] = np.repeat(np.arange(self.n), count)
+                q[:, 2] = 32 * rows * (np.arange(len(q)) - np.repeat(np.cumsum(count) - count, count))
+                parts.append(q)
+            for b, (nx, ny) in enumerate(self.sizes if not flat else ()):
                 v = self.vw if (vector and ny % self.vw == 0) else 1
                 ks = np.arange(0, nx, rows, dtype=np.int32)
                 zs = np.arange(0, ny, 32 * v, dtype=np.int32)
@@ -216,7 +216,7 @@ class BatchedLattice:
             self._slice(int(b), other).copy_(self._slice(int(b)))
         self.active = mask
         self._tasks = {k: v for k, v in self._tasks.items() if k[3] is None}
-        self._step_tasks = {k: v for k, v in self._step_tasks.items() if k[1] is None}
+        self._step_tasks = {k: v for k, v in self._step_tasks.items() if k is None}
 
     def _queue(self, cfg):
         flat = bool(cfg.get("flat", False))
@@ -241,19 +241,21 @@ class BatchedLattice:
                   cfg["blocks"], int(flat), self._stream())
 
     # ------------------------------------------------------------ several steps per launch
-    def _plan(self, steps=0):
-        """(kind, most steps of a launch, host task list of a launch of ``steps`` steps) of lbgb_batch_plan."""
+    def _plan(self, steps=None):
+        """(kind, most steps of a launch, host task list of a launch of ``steps``
+        steps, empty for None) of lbgb_batch_plan."""
         nx = np.ascontiguousarray(self._table_np["nx"])
         ny = np.ascontiguousarray(self._table_np["ny"])
         kind, most, count = ctypes.c_int(0), ctypes.c_int(1), ctypes.c_longlong(0)
-        tasks = np.zeros((0, 4), dtype=np.int32)
+        # room for the tasks of most batches: one call
+        tasks = np.empty((0 if steps is None else 1024 + 32 * self.n, 4), dtype=np.int32)
         while True:
-            _lib.call("lbgb_batch_plan", nx.ctypes.data, ny.ctypes.data, self.n, self.bcode, self.code, int(steps),
-                      ctypes.byref(kind), ctypes.byref(most), tasks.ctypes.data if len(tasks) else None, len(tasks),
-                      ctypes.byref(count))
-            if len(tasks) == count.value:
-                return kind.value, most.value, tasks
-            tasks = np.zeros((count.value, 4), dtype=np.int32)
+            _lib.call("lbgb_batch_plan", nx.ctypes.data, ny.ctypes.data, self.n, self.bcode, self.code,
+                      int(steps or 0), ctypes.byref(kind), ctypes.byref(most), tasks.ctypes.data if len(tasks) else None,
+                      len(tasks), ctypes.byref(count))
+            if steps is None or count.value <= len(tasks):
+                return kind.value, most.value, tasks[:count.value]
+            tasks = np.empty((count.value, 4), dtype=np.int32)
 
     def _several(self):
         key = int(_lib.get_tuning(_lib.TUNE_TWO_STEP))
@@ -276,18 +278,33 @@ class BatchedLattice:
             left -= t
         return kind, several, left
 
-    def _launch_steps(self, kind, t):
+    def _mask(self):
+        return None if self.active.all() else self.active.tobytes()
+
+    def _ready(self, kind, most):
+        """{steps: task list} of the launches that any number of steps of the
+        active instances takes.  All of them, and what single steps need, go to
+        the device at the first one, so that a caller may capture steps in a
+        graph after a warm-up of other lengths."""
+        mask = self._mask()
+        cfg = self.config
+        if kind == _lib.BATCH_MARCH and (bool(cfg["vector"]), int(cfg["rows"]), bool(cfg.get("flat", False)),
+                                         mask) not in self._tasks:
+            self._queue(cfg)  # the march leaves a last odd step
+            self._table(cfg["vector"])
+        lists = self._step_tasks.get(mask)
+        if lists is None:
+            self._table(True)
+            steps = range(1, most + 1) if kind == _lib.BATCH_TILE else (2, 4)
+            host = [self._plan(t)[2] for t in steps]
+            if mask is not None:
+                host = [q[self.active[q[:, 0]]] for q in host]
+            tasks = torch.from_numpy(np.concatenate(host)).to(self.device)
+            lists = self._step_tasks[mask] = dict(zip(steps, tasks.split([len(q) for q in host])))
+        return lists
+
+    def _launch_steps(self, kind, t, tasks):
         """One launch of t steps of the active instances."""
-        full = self._step_tasks.get((t, None))
-        if full is None:
-            full = self._step_tasks[(t, None)] = torch.from_numpy(self._plan(t)[2]).to(self.device)
-        tasks = full
-        if not self.active.all():
-            key = (t, self.active.tobytes())
-            tasks = self._step_tasks.get(key)
-            if tasks is None:
-                keep = torch.from_numpy(self.active).to(self.device)[full[:, 0].long()]
-                tasks = self._step_tasks[key] = full[keep].contiguous()
         src, dst = self._buf[self._cur], self._buf[1 - self._cur]
         if tasks.shape[0] == 0:
             dst.copy_(src)
@@ -301,8 +318,10 @@ class BatchedLattice:
         lbgb_batch_plan; the same results bit for bit), or one per launch of
         ``config`` where one is given or several do not apply."""
         kind, several, singles = self._schedule(int(n)) if config is None else (None, [], int(n))
+        if several or kind == _lib.BATCH_MARCH:
+            lists = self._ready(kind, self._several()[1])
         for t in several:
-            self._launch_steps(kind, t)
+            self._launch_steps(kind, t, lists[t])
         cfg = config or self.config
         for _ in range(singles):
             self._launch(self._buf[self._cur], self._buf[1 - self._cur], cfg)

@@ -67,3 +67,24 @@ def test_state_loaded_between_replays(two_step, cuda):
     replay()
     ref.step(2)
     assert torch.equal(lat.state, ref.state)
+
+
+@pytest.mark.parametrize("sizes", [SMALL, LARGE])
+@pytest.mark.parametrize("retired", [False, True])
+def test_batch_in_a_graph_of_the_callers(cuda, sizes, retired):
+    """After a warm-up of two steps any number of steps can be captured."""
+    a, b = make(sizes, "f32", "periodic", cuda), make(sizes, "f32", "periodic", cuda)
+    if retired:
+        for x in (a, b):
+            x.set_active(np.arange(len(sizes)) % 3 != 1)
+    a.step(2)
+    b.step(2, SINGLE)
+    for n in (10, 3, 1, 8, 5):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            a.step(n)
+        g.replay()
+        b.step(n, SINGLE)
+        torch.cuda.synchronize()
+        for i in range(len(sizes)):
+            assert torch.equal(a.populations(i), b.populations(i))
