@@ -301,6 +301,7 @@ class FNO2d:
                 flat, rows = (_lib.load().lbgb_fno_layer_sums(*x) for x in ((1, N, 0), (B * H, W, m2)))
                 ws["df"] = None if flat and rows else torch.empty(C if flat else max(self.hidden, C), N, **f32)
                 ws["flat_sums"], ws["row_sums"] = flat, rows
+                ws["q1"], ws["q1b"] = torch.empty(self.hidden * C, **bf), torch.empty(self.hidden, **f32)
             else:
                 ws.update({"dh": torch.empty(self.hidden, N, **f32), "dv": torch.empty(C, N, **f32)})
         self._ws[key] = ws
@@ -392,7 +393,11 @@ class FNO2d:
         _lib.call("lbgb_fno_project", self.hidden, C, 1, N, _ptr(at(self.layers)), _ptr(pb, o["Q1"]),
                   _ptr(fl, o["q1b"]), self.cout, _ptr(pb, o["Q2"]), _ptr(fl, o["q2b"]),
                   _ptr(ws["gb"]) if train else None, None if train else _ptr(ws["out"]), s)
-        if train:  # the loss gradient is rounded to BF16: the output in the order of the other engines
+        if train:
+            # backward computes the hidden layer again: with the parameters it had here
+            ws["q1"].copy_(pb[o["Q1"]:o["Q1"] + self.hidden * C])
+            ws["q1b"].copy_(fl[o["q1b"]:o["q1b"] + self.hidden])
+            # the loss gradient is rounded to BF16: the output in the order of the other engines
             self._outputs(ws, N)
         return ws["out"].view(self.cout, B, H, W)
 
@@ -424,8 +429,7 @@ class FNO2d:
         return loss
 
     def backward(self, d):
-        """Gradients from d = dLoss/dout (cout, N) FP32 of the last training forward
-        (with the parameters it ran with)."""
+        """Gradients from d = dLoss/dout (cout, N) FP32 of the last training forward."""
         B, H, W = self._shape
         N = B * H * W
         ws = self._ws[(B, H, W, True, self._fused(B, H, W))]
@@ -490,12 +494,12 @@ class FNO2d:
         fw, _, _, Gt, _ = self.matrices(H, W)
         C, m, hid, L, N = self.width, self.modes, self.hidden, self.layers, B * H * W
         q2, m2 = 4 * m, 2 * m
-        s, pb, fl, g, o = self._s(), self.flat_bf16, self.flat, self.grad, self.offsets
+        s, pb, g, o = self._s(), self.flat_bf16, self.grad, self.offsets
         sums, dhb, vb = _ptr(ws["sums"]), _ptr(ws["dhb"]), ws["vb"]
         dz, other = ws["dzb"]
         f32 = _ptr(ws["df"]) if ws["df"] is not None else None
         flat, rows = None if ws["flat_sums"] else f32, None if ws["row_sums"] else f32
-        _lib.call("lbgb_fno_project_back", hid, C, 1, N, _ptr(vb[L]), _ptr(pb, o["Q1"]), _ptr(fl, o["q1b"]), self.cout,
+        _lib.call("lbgb_fno_project_back", hid, C, 1, N, _ptr(vb[L]), _ptr(ws["q1"]), _ptr(ws["q1b"]), self.cout,
                   _ptr(pb, o["Q2"]), _ptr(ws["db"]), dhb, flat, _ptr(g, o["q1b"]), sums, s)
         self._wgrad(hid, C, N, dhb, _ptr(vb[L]), _ptr(g, o["Q1"]), C, 1, ws)
         # the gradient of each layer's z, from the last layer's (no activation) down
