@@ -119,6 +119,7 @@ class FNO2d:
         self.adam_steps = 0
         self.out_scale = np.ones(cout)  # network output c is target channel c / out_scale[c]
         self._mats, self._ws = {}, {}
+        self._train_form = {}  # (B, H, W) -> whether its last training forward ran the fused layers
         self.init_params(np.random.default_rng(seed))
 
     # ------------------------------------------------------------ parameters
@@ -266,6 +267,7 @@ class FNO2d:
         # keep at most a couple of shapes alive
         if len(self._ws) > 2:
             self._ws.clear()
+            self._train_form.clear()
         N = B * H * W
         C, L, m = self.width, self.layers, self.modes
         q2, m2 = 4 * m, 2 * m
@@ -316,13 +318,16 @@ class FNO2d:
         N = B * H * W
         ws = self._workspace(B, H, W, train)
         self._shape = (B, H, W)
+        fused = self._fused(B, H, W)
+        if train:
+            self._train_form[self._shape] = fused
         _, _, iw, _, _ = self.matrices(H, W)
         C, m = self.width, self.modes
         q2, m2 = 4 * m, 2 * m
         s = self._s()
         pb = self.flat_bf16
         _lib.call("lbgb_fno_to_bf16", a.data_ptr(), ws["ab"].data_ptr(), a.numel(), s)
-        if self._fused(B, H, W):
+        if fused:
             return self._forward_fused(ws, B, H, W, train)
         z0 = ws["z"][0]
         # lifting: v0 = P a + p
@@ -410,7 +415,7 @@ class FNO2d:
         out = self.forward(a, train=True)
         B, H, W = self._shape
         N = B * H * W
-        ws = self._ws[(B, H, W, True, self._fused(B, H, W))]
+        ws = self._ws[(B, H, W, True, self._train_form[self._shape])]
         if target.shape != out.shape or target.dtype != torch.float32 or not target.is_contiguous():
             raise ValueError("target must be a contiguous float32 tensor of shape %s" % (tuple(out.shape),))
         s = self._s()
@@ -432,7 +437,8 @@ class FNO2d:
         """Gradients from d = dLoss/dout (cout, N) FP32 of the last training forward."""
         B, H, W = self._shape
         N = B * H * W
-        ws = self._ws[(B, H, W, True, self._fused(B, H, W))]
+        fused = self._train_form[self._shape]
+        ws = self._ws[(B, H, W, True, fused)]
         fw, _, _, Gt, _ = self.matrices(H, W)
         C, m, hid = self.width, self.modes, self.hidden
         q2, m2 = 4 * m, 2 * m
@@ -443,7 +449,7 @@ class FNO2d:
         # out = Q2 g + q2
         self._wgrad(hid, self.cout, N, _ptr(ws["gb"]), _ptr(ws["db"]), _ptr(g, o["Q2"]), 1, hid, ws)
         _lib.call("lbgb_fno_row_sum", _ptr(d), _ptr(g, o["q2b"]), _ptr(ws["rowsum"]), self.cout, N, s)
-        if self._fused(B, H, W):
+        if fused:
             self._backward_fused(ws, B, H, W)
             return
         dh = ws["dh"]

@@ -1,5 +1,5 @@
-"""Gradients belong to the last training forward, also if the parameters are
-changed between it and backward.  Reference: the network
+"""Gradients belong to the last training forward, whatever is changed between it
+and backward: the parameters, or how the layers run.  Reference: the network
 that runs one pass per operation and keeps the hidden layer's values, whose
 gradients the fused one equals bit for bit."""
 
@@ -36,6 +36,23 @@ def test_parameters_changed_before_backward(cuda):
         net.backward(d)
         out.append(grads(net))
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("first", [True, False])
+def test_form_switched_before_backward(cuda, first):
+    net, a, d = net_and_inputs(cuda, first)
+    net.forward(a, train=True)
+    net.backward(d)
+    before = grads(net)
+    net.forward(a, train=True)
+    net.grad.zero_()
+    net.fused_epilogue = not first
+    net.backward(d)
+    assert torch.equal(grads(net), before)
+    net.forward(a)  # of the other form, without gradients
+    net.grad.zero_()
+    net.backward(d)
+    assert torch.equal(grads(net), before)
 
 
 def test_backward_needs_a_training_forward(cuda):
