@@ -25,6 +25,7 @@
 #include "lbgb_common.cuh"
 #include "lbgb_march.h"
 #include "lbgb_pipe.cuh"
+#include "lbgb_run.h"
 #include "lbgb_tile.h"
 
 namespace lbgb {
@@ -557,16 +558,19 @@ extern "C" int lbgb_run_fused(void *a, void *b, int nx, int ny, int boundary, do
     if (rc) return rc;
     void *src = a, *dst = b;
     const Several m = several_steps(a, b, nx, ny, dtype, false);
-    for (int left = nsteps; left > 0;) {
-        const int n = next_steps(m, left);
-        rc = n > 1 ? several(m, src, dst, nx, ny, boundary, omega, u0, dtype, n, SR(), (cudaStream_t)stream)
-                   : lbgb_step_fused(src, dst, nx, ny, boundary, omega, u0, dtype, stream);
-        if (rc) return rc;
-        left -= n;
-        void *t = src;
-        src = dst;
-        dst = t;
-    }
+    int done;
+    rc = run_steps(
+        nsteps, [&](int left) { return next_steps(m, left); },
+        [&](int n, int) {
+            const int e = n > 1 ? several(m, src, dst, nx, ny, boundary, omega, u0, dtype, n, SR(), (cudaStream_t)stream)
+                                : lbgb_step_fused(src, dst, nx, ny, boundary, omega, u0, dtype, stream);
+            void *t = src;
+            src = dst;
+            dst = t;
+            return e;
+        },
+        &done);
+    if (rc) return rc;
     if (which) *which = (src == a) ? 0 : 1;
     return LBGB_OK;
 }
@@ -610,26 +614,26 @@ extern "C" int lbgb_run_fused_sr(void *a, void *b, int nx, int ny, int boundary,
     sr.seed = seed;
     void *src = a, *dst = b;
     const Several m = several_steps(a, b, nx, ny, dtype, true);
-    for (int left = nsteps; left > 0;) {
-        const int n = next_steps(m, left);
-        sr.offset = (uint32_t)(nsteps - left);
-        rc = n > 1 ? several(m, src, dst, nx, ny, boundary, omega, u0, dtype, n, sr, s)
-             : boundary == LBGB_CAVITY
-                 ? dispatch<LBGB_CAVITY, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
-             : boundary == LBGB_CAVITY_LADD
-                 ? dispatch<LBGB_CAVITY_LADD, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
-                 : dispatch<LBGB_PERIODIC, true>(src, dst, nx, ny, dtype, omega, 0.0, s, sr);
-        if (rc) return rc;
-        left -= n;
-        void *t = src;
-        src = dst;
-        dst = t;
-    }
-    if (nsteps > 0) {
-        k_bump_step<<<1, 1, 0, s>>>(step_counter, (unsigned long long)nsteps);
-        rc = check_launch("k_bump_step");
-        if (rc) return rc;
-    }
+    rc = run_counted_steps(
+        nsteps, [&](int left) { return next_steps(m, left); },
+        [&](int n, int done) {
+            sr.offset = (uint32_t)done;
+            const int e = n > 1 ? several(m, src, dst, nx, ny, boundary, omega, u0, dtype, n, sr, s)
+                          : boundary == LBGB_CAVITY
+                              ? dispatch<LBGB_CAVITY, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
+                          : boundary == LBGB_CAVITY_LADD
+                              ? dispatch<LBGB_CAVITY_LADD, true>(src, dst, nx, ny, dtype, omega, u0, s, sr)
+                              : dispatch<LBGB_PERIODIC, true>(src, dst, nx, ny, dtype, omega, 0.0, s, sr);
+            void *t = src;
+            src = dst;
+            dst = t;
+            return e;
+        },
+        [&](int n) {
+            k_bump_step<<<1, 1, 0, s>>>(step_counter, (unsigned long long)n);
+            return check_launch("k_bump_step");
+        });
+    if (rc) return rc;
     if (which) *which = (src == a) ? 0 : 1;
     return LBGB_OK;
 }
