@@ -237,62 +237,66 @@ __global__ void __launch_bounds__(128) k_mix_bwd_x(const float *__restrict__ dYm
 constexpr int MIXR_K = 16, MIXR_C = 4, MIXR_O = 32, MIXR_B = 8, MIXR_T = 16;
 
 __global__ void k_mix_bwd_r(const float *__restrict__ dYm, const float *__restrict__ P, float *__restrict__ dRr,
-                            float *__restrict__ dRi, int C, int O, int B, int q, int mk, int kt) {
+                            float *__restrict__ dRi, int C, int O, int B, int q, int mk, int kt,
+                            long long units) {
     extern __shared__ float2 mix_sm[];  // x [MIXR_C][MIXR_B][kt], then dy [MIXR_O][MIXR_B][kt]
     float2 *sx = mix_sm, *sg = mix_sm + MIXR_C * MIXR_B * kt;
-    const int Q = q * mk, y = blockIdx.x % q, k0 = blockIdx.x / q * kt;
-    const int o0 = blockIdx.y * MIXR_O, c0 = blockIdx.z * MIXR_C;
+    const int Q = q * mk, kts = (mk + kt - 1) / kt, ots = (O + MIXR_O - 1) / MIXR_O;
     const long long pcb = 4LL * mk * q;
     const int k = threadIdx.x % kt, og = threadIdx.x / kt;  // this thread's kx and every MIXR_T-th o from og
     constexpr int NO = MIXR_O / MIXR_T;
-    float ar[MIXR_C][NO] = {}, ai[MIXR_C][NO] = {};
-    for (int b0 = 0; b0 < B; b0 += MIXR_B) {
-        const int nb = min(MIXR_B, B - b0);
+    // unit: ky fastest, then the kx, the outputs and the inputs a block takes
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        const int y = (int)(u % q), k0 = (int)(u / q % kts) * kt;
+        const int o0 = (int)(u / q / kts % ots) * MIXR_O, c0 = (int)(u / q / kts / ots) * MIXR_C;
+        float ar[MIXR_C][NO] = {}, ai[MIXR_C][NO] = {};
+        for (int b0 = 0; b0 < B; b0 += MIXR_B) {
+            const int nb = min(MIXR_B, B - b0);
 #pragma unroll 3
-        for (int e = og; e < (MIXR_C + MIXR_O) * nb; e += MIXR_T) {
-            const int ch = e / nb, b = e - ch * nb;
-            const bool is_x = ch < MIXR_C;
-            const int c = is_x ? c0 + ch : o0 + ch - MIXR_C;
-            float2 v = make_float2(0.f, 0.f);
-            if (k0 + k < mk && c < (is_x ? C : O)) {
-                if (is_x)
-                    mode_x(P + ((long long)c * B + b0 + b) * pcb, y, k0 + k, q, mk, v.x, v.y);
-                else
-                    mode_dy(dYm + ((long long)c * B + b0 + b) * pcb, y, k0 + k, q, mk, v.x, v.y);
+            for (int e = og; e < (MIXR_C + MIXR_O) * nb; e += MIXR_T) {
+                const int ch = e / nb, b = e - ch * nb;
+                const bool is_x = ch < MIXR_C;
+                const int c = is_x ? c0 + ch : o0 + ch - MIXR_C;
+                float2 v = make_float2(0.f, 0.f);
+                if (k0 + k < mk && c < (is_x ? C : O)) {
+                    if (is_x)
+                        mode_x(P + ((long long)c * B + b0 + b) * pcb, y, k0 + k, q, mk, v.x, v.y);
+                    else
+                        mode_dy(dYm + ((long long)c * B + b0 + b) * pcb, y, k0 + k, q, mk, v.x, v.y);
+                }
+                (is_x ? sx + ch * MIXR_B * kt : sg + (ch - MIXR_C) * MIXR_B * kt)[b * kt + k] = v;
             }
-            (is_x ? sx + ch * MIXR_B * kt : sg + (ch - MIXR_C) * MIXR_B * kt)[b * kt + k] = v;
-        }
-        __syncthreads();
-        for (int b = 0; b < nb; ++b) {
-            float2 g[NO];
+            __syncthreads();
+            for (int b = 0; b < nb; ++b) {
+                float2 g[NO];
 #pragma unroll
-            for (int i = 0; i < NO; ++i) g[i] = sg[((og + i * MIXR_T) * MIXR_B + b) * kt + k];
+                for (int i = 0; i < NO; ++i) g[i] = sg[((og + i * MIXR_T) * MIXR_B + b) * kt + k];
 #pragma unroll
-            for (int h = 0; h < MIXR_C; ++h) {
-                const float2 x = sx[(h * MIXR_B + b) * kt + k];
-                const float xr = x.x, xi = x.y;
+                for (int h = 0; h < MIXR_C; ++h) {
+                    const float2 x = sx[(h * MIXR_B + b) * kt + k];
+                    const float xr = x.x, xi = x.y;
 #pragma unroll
-                for (int i = 0; i < NO; ++i) {
-                    const float gr = g[i].x, gi = g[i].y;
-                    ar[h][i] += gr * xr + gi * xi;
-                    ai[h][i] += -gr * xi + gi * xr;
+                    for (int i = 0; i < NO; ++i) {
+                        const float gr = g[i].x, gi = g[i].y;
+                        ar[h][i] += gr * xr + gi * xi;
+                        ai[h][i] += -gr * xi + gi * xr;
+                    }
                 }
             }
+            __syncthreads();
         }
-        __syncthreads();
-    }
-    if (k0 + k >= mk) return;
 #pragma unroll
-    for (int h = 0; h < MIXR_C; ++h)
+        for (int h = 0; h < MIXR_C; ++h)
 #pragma unroll
-        for (int i = 0; i < NO; ++i) {
-            const int c = c0 + h, o = o0 + og + i * MIXR_T;
-            if (c < C && o < O) {
-                const long long r = ((long long)c * O + o) * Q + y * mk + k0 + k;
-                dRr[r] = ar[h][i];
-                dRi[r] = ai[h][i];
+            for (int i = 0; i < NO; ++i) {
+                const int c = c0 + h, o = o0 + og + i * MIXR_T;
+                if (k0 + k < mk && c < C && o < O) {
+                    const long long r = ((long long)c * O + o) * Q + y * mk + k0 + k;
+                    dRr[r] = ar[h][i];
+                    dRi[r] = ai[h][i];
+                }
             }
-        }
+    }
 }
 
 // mean squared error: partial sums per block into part[], and d = 2 (y - t) / n
@@ -476,13 +480,11 @@ extern "C" int lbgb_fno_mix_back(const float *dYm, const float *P, const void *R
         static_cast<__nv_bfloat16 *>(dP), C, O, B, q, mk);
     int rc = check_launch("k_mix_bwd_x");
     if (rc) return rc;
-    const int kt = mk < MIXR_K ? mk : MIXR_K, ot = (O + MIXR_O - 1) / MIXR_O, ct = (C + MIXR_C - 1) / MIXR_C;
-    if (ot > 65535 || ct > 65535 || (long long)q * ((mk + kt - 1) / kt) > 2147483647ll) {
-        set_error("lbgb_fno_mix_back: too many channels or modes");
-        return LBGB_EINVAL;
-    }
+    const int kt = mk < MIXR_K ? mk : MIXR_K;
+    const long long units = (long long)q * ((mk + kt - 1) / kt) * ((O + MIXR_O - 1) / MIXR_O) * ((C + MIXR_C - 1) / MIXR_C);
+    const unsigned grid = (unsigned)(units < 2147483647ll ? units : 2147483647ll);
     const size_t smem = sizeof(float2) * (MIXR_C + MIXR_O) * MIXR_B * kt;
-    k_mix_bwd_r<<<dim3(q * ((mk + kt - 1) / kt), ot, ct), kt * MIXR_T, smem, s>>>(dYm, P, dRr, dRi, C, O, B, q, mk, kt);
+    k_mix_bwd_r<<<grid, kt * MIXR_T, smem, s>>>(dYm, P, dRr, dRi, C, O, B, q, mk, kt, units);
     return check_launch("k_mix_bwd_r");
 }
 
