@@ -441,6 +441,7 @@ LBGB_API int lbgb_fno_mix_back(const float *dYm, const float *P, const void *Rr,
  *                 rounding; n <= 32
  *   project       h = x q1 + q1b, g = BF16(gelu(h)) (null: not stored), out (cout <= 4, rows * w) =
  *                 q2 g + q2b (null: not computed); n <= 128 hidden channels
+ *   hidden        project's g alone, and copies of the q1 (n, k1) and q1b (n) used
  *   project_back  dh = BF16((q2^T d) gelu'(h)), d BF16 (cout <= 64, rows * w), with h computed
  *                 again; sums as above
  * The sums are lbgb_fno_row_sum's, addition for addition; f32 (n, rows * w), 16-byte
@@ -454,6 +455,8 @@ LBGB_API int lbgb_fno_layer_back(int n, int k1, int rows, int w, const void *x, 
                                  float *f32, float *sums, float *parts, void *stream);
 LBGB_API int lbgb_fno_project(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
                               int cout, const void *q2, const float *q2b, void *g, float *out, void *stream);
+LBGB_API int lbgb_fno_hidden(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b, void *g,
+                             void *q1_copy, float *q1b_copy, void *stream);
 LBGB_API int lbgb_fno_project_back(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
                                    int cout, const void *q2, const void *d, void *dh, float *f32, float *sums,
                                    float *parts, void *stream);

@@ -94,6 +94,7 @@ SIGNATURES = {
     "lbgb_fno_layer_back": (_I, [_I, _I, _I, _I, _P, _P, ctypes.c_longlong, ctypes.c_longlong, _I, _P, _P, _P, _P, _P,
                                  _P, _P, _P]),
     "lbgb_fno_project": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _P]),
+    "lbgb_fno_hidden": (_I, [_I, _I, _I, _I, _P, _P, _P, _P, _P, _P, _P]),
     "lbgb_fno_project_back": (_I, [_I, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P]),
     "lbgb_fno_layer_parts": (ctypes.c_longlong, [_I]),
     "lbgb_fno_layer_sums": (_I, [_I, _I, _I]),

@@ -1091,6 +1091,20 @@ extern "C" int lbgb_fno_project(int n, int k1, int rows, int w, const void *x, c
     return launch_layer<PROJECT>(a, x, nullptr, nullptr, nullptr, (cudaStream_t)stream, "lbgb_fno_project");
 }
 
+extern "C" int lbgb_fno_hidden(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b, void *g,
+                               void *q1_copy, float *q1b_copy, void *stream) {
+    if (!x || !q1 || !q1b || !g || !aligned(g, 16) || !q1_copy || !q1b_copy || !aligned(q1_copy, 2)) {
+        set_error("lbgb_fno_hidden: null or misaligned operand");
+        return LBGB_EINVAL;
+    }
+    LayerArgs a{};
+    a.n = n, a.k1 = k1, a.rows = rows, a.W = w;
+    a.b1 = static_cast<const __nv_bfloat16 *>(q1), a.b1_ns = k1, a.b1_ks = 1;
+    a.bias = q1b, a.v = static_cast<__nv_bfloat16 *>(g);
+    a.b1_copy = static_cast<__nv_bfloat16 *>(q1_copy), a.bias_copy = q1b_copy;
+    return launch_layer<HIDDEN>(a, x, nullptr, nullptr, nullptr, (cudaStream_t)stream, "lbgb_fno_hidden");
+}
+
 extern "C" int lbgb_fno_project_back(int n, int k1, int rows, int w, const void *x, const void *q1, const float *q1b,
                                      int cout, const void *q2, const void *d, void *dh, float *f32, float *sums,
                                      float *parts, void *stream) {

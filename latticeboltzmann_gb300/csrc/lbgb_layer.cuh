@@ -68,6 +68,8 @@ struct LayerArgs {
     const float *q2b;
     int cout;
     float *out;                    // PROJECT: (cout, rows * W)
+    __nv_bfloat16 *b1_copy;        // HIDDEN: (n, k1) b1 and (n) bias as used, or null
+    float *bias_copy;
 };
 
 // The sums over the pixels add in the order of lbgb_fno_row_sum, so that a
@@ -194,6 +196,7 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         const int n = e / (kb1 * 64), k = e - n * (kb1 * 64);
         const __nv_bfloat16 x = n < a.n && k < a.k1 ? a.b1[n * a.b1_ns + k * a.b1_ks] : __float2bfloat16_rn(0.f);
         *reinterpret_cast<__nv_bfloat16 *>(sb1 + b1_offset(NT, n, k)) = x;
+        if (MODE == HIDDEN && a.b1_copy && blockIdx.x == 0 && n < a.n && k < a.k1) a.b1_copy[n * a.k1 + k] = x;
     }
     unsigned char *sq2 = sb1 + kb1 * NT * 128;
     if (MODE == PROJECT_BACK)
@@ -204,6 +207,7 @@ k_layer(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtenso
         }
     for (int c = threadIdx.x; c < NT; c += S::THREADS) {
         s_bias[c] = a.bias && c < a.n ? a.bias[c] : 0.f;
+        if (MODE == HIDDEN && a.bias_copy && blockIdx.x == 0 && c < a.n) a.bias_copy[c] = s_bias[c];
         if (MODE == PROJECT) {
             float q[4] = {0.f, 0.f, 0.f, 0.f};
             for (int o = 0; o < 4; ++o)

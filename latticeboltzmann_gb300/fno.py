@@ -395,15 +395,15 @@ class FNO2d:
             _lib.call("lbgb_fno_layer", C, C, B * H, W, _ptr(at(l)), _ptr(pb, o["W%d" % l]), C, 1, m2, _ptr(iwt),
                       _ptr(ws["Z"]), _ptr(fl, o["b%d" % l]), int(not last),
                       _ptr(ws["z"][l]) if train and not last else None, _ptr(at(l + 1)), s)
-        _lib.call("lbgb_fno_project", self.hidden, C, 1, N, _ptr(at(self.layers)), _ptr(pb, o["Q1"]),
-                  _ptr(fl, o["q1b"]), self.cout, _ptr(pb, o["Q2"]), _ptr(fl, o["q2b"]),
-                  _ptr(ws["gb"]) if train else None, None if train else _ptr(ws["out"]), s)
+        hidden = (self.hidden, C, 1, N, _ptr(at(self.layers)), _ptr(pb, o["Q1"]), _ptr(fl, o["q1b"]))
         if train:
-            # backward computes the hidden layer again: with the parameters it had here
-            ws["q1"].copy_(pb[o["Q1"]:o["Q1"] + self.hidden * C])
-            ws["q1b"].copy_(fl[o["q1b"]:o["q1b"] + self.hidden])
+            # backward computes the hidden layer again: with the parameters it has here
+            _lib.call("lbgb_fno_hidden", *hidden, _ptr(ws["gb"]), _ptr(ws["q1"]), _ptr(ws["q1b"]), s)
             # the loss gradient is rounded to BF16: the output in the order of the other engines
             self._outputs(ws, N)
+        else:
+            _lib.call("lbgb_fno_project", *hidden, self.cout, _ptr(pb, o["Q2"]), _ptr(fl, o["q2b"]), None,
+                      _ptr(ws["out"]), s)
         return ws["out"].view(self.cout, B, H, W)
 
     def loss_and_backward(self, a, target, weight=None):
