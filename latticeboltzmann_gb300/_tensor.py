@@ -30,16 +30,24 @@ def storage_code(t, name):
         raise TypeError("%s: dtype %s not supported (float32 or float64)" % (name, t.dtype)) from None
 
 
+def _stream_of_index(index):
+    return torch.cuda.current_stream(index).cuda_stream
+
+
+# Handle of a device's current stream without the stream object, whose making
+# takes a fifth of a small operator's host time; torch versions without that
+# query make the object.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _stream_of_index)
+
+
 def stream_of(device):
-    """Handle of the device's current stream: ``torch.cuda.current_stream(device)
-    .cuda_stream`` without the stream object, whose making takes a fifth of a
-    small operator's host time."""
+    """Handle of the device's current stream."""
     index = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def stream_handle(t):
-    return torch._C._cuda_getCurrentRawStream(t.get_device())
+    return _raw_stream(t.get_device())
 
 
 def population_view(f, name):
