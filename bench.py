@@ -207,24 +207,36 @@ def hbm_peak():
 
 
 def steps_per_event(lat, steps):
-    """The most steps that one launch advances, of those that divide ``steps``."""
+    """The most steps that one launch advances, of those that divide ``steps``.
+    (Where the most is 4 the kernel may be the march, which takes 4, 2 or 1;
+    tiles take any number.)"""
     from latticeboltzmann_gb300 import _lib
     most = int(_lib.load().lbgb_max_steps_per_launch(lat.nx, lat.ny, lat.bcode, lat.code))
-    return next(c for c in range(most, 0, -1) if steps % c == 0)
+    return next(c for c in range(most, 0, -1) if steps % c == 0 and (most, c) != (4, 3))
 
 
-def profiled_traffic(storage, boundary, cells, kernel="k_step_pipe"):
-    """DRAM bytes per launch of the fused kernel from the committed ncu summary,
-    scaled from the captured grid to ``cells`` (traffic is proportional to cells)."""
-    path = os.path.join(ROOT, "profiles", "k_step_traffic.json")
-    try:
-        with open(path) as fh:
-            rows = json.load(fh)
-    except (OSError, ValueError):
-        return None, None
+def step_kernel(cells, steps):
+    """The kernel of a launch of ``steps`` steps: marches begin at 0.95 M cells
+    (FP32), tiles of rows without whole vectors go on beyond."""
+    if steps == 1:
+        return "k_step_pipe"
+    return "k_march" if steps in (2, 4) and cells >= 1500000 else "k_march / k_tile"
+
+
+def profiled_traffic(storage, boundary, cells, kernel="k_step_pipe", steps=None):
+    """DRAM bytes per launch of the fused kernel from the committed ncu summaries,
+    scaled from the captured grid to ``cells`` (traffic is proportional to cells).
+    ``steps``: steps of the launch, where the kernel takes several numbers."""
+    rows = []
+    for name in ("k_step_traffic.json", "k_march_traffic.json"):
+        try:
+            with open(os.path.join(ROOT, "profiles", name)) as fh:
+                rows += json.load(fh)
+        except (OSError, ValueError):
+            pass
     for r in rows:
-        if (r.get("storage") == storage and r.get("boundary") == boundary
-                and r.get("kernel", "k_step_pipe") == kernel):
+        if (r.get("storage") == storage and r.get("boundary") == boundary and r.get("kernel", "k_step_pipe") == kernel
+                and (steps is None or r.get("steps_per_launch", 1) == steps)):
             return r["dram_bytes_per_launch"] * cells / r["cells"], r
     return None, None
 
@@ -474,14 +486,14 @@ def run_ours(args):
     avg_launch_s = sum(per_launch_ms) / len(per_launch_ms) / 1e3
     achieved = bpc * lat.cells / avg_launch_s / 1e9
     peak, peak_src = hbm_peak()
-    kname = "k_march" if chunk > 1 else "k_step_pipe"
-    traffic, prof = profiled_traffic(args.storage, args.boundary, lat.cells, kname)
+    kname = step_kernel(lat.cells, chunk)
+    traffic, prof = profiled_traffic(args.storage, args.boundary, lat.cells, kname, chunk)
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": None if traffic is None else round(traffic),
                 "algorithmic_bytes": bpc * lat.cells, "steps_per_launch": chunk,
                 "bytes_per_cell_update": bpc / chunk,
-                "kernel": ("k_march / k_tile (%d fused steps per launch: pull stream + bounce-back/lid + BGK, the "
-                           "intermediate steps on chip)" % chunk if chunk > 1 else
+                "kernel": ("%s (%d fused steps per launch: pull stream + bounce-back/lid + BGK, the "
+                           "intermediate steps on chip)" % (kname, chunk) if chunk > 1 else
                            "k_step (fused pull stream + bounce-back/lid + BGK)"),
                 "peak_source": peak_src,
                 "traffic_source": None if prof is None else prof.get("source")}
