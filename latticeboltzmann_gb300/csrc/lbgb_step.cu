@@ -282,7 +282,7 @@ struct Tuning {
     long long wait_limit = 1ll << 22;    // tries per bounded mbarrier wait
     long long pipe_min_cells = 1 << 16;  // auto: smaller lattices use the register kernel
     long long stall_producer = 0;        // test hook: the producer delivers nothing
-    long long two_step = 1;              // auto kernel: several time steps per launch where k_march applies
+    long long two_step = 1;              // auto kernel: several time steps per launch where k_tile or k_march applies
 };
 static Tuning g_tune;
 

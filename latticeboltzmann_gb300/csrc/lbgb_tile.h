@@ -110,10 +110,12 @@ inline void tile_plan(TilePlan &p, int nx, int ny, int kind, int element, double
 
 // Expected SM cycles of one step in a launch of its own, rows of whole vectors:
 // 5800 for the launch and 0.0205 a cell over 152 SMs (94,000 MLUPS), 16-bit codes
-// 0.0154.  Lattices two to five rows high have tiles that are mostly halo, and
-// one step per launch is faster (2 x 400,000 FP32 12.3 us against 19.3, half 9.9
-// against 15.4; 5 x 200,000 half 10.3 against 13.6).  Rows without whole vectors
-// are slower one step at a time than any tile; FP64 differs by a tenth at most.
+// 0.0154.  Tiles of long lattices a few rows high are mostly halo: one step per
+// launch is faster below 8 rows (2 x 400,000 FP32 12.3 us against 19.3, half 9.9
+// against 15.4; 5 x 200,000 half 10.3 against 13.6), the march of two steps from
+// there on (8 x 112,496 stochastic half 8.5 us against 13.2, 16 x 56,248 8.4
+// against 12.5).  Rows without whole vectors are slower one step at a time than
+// any tile; FP64 differs by a tenth at most.
 inline double single_cost(double cells, int element, int sms) {
     return 5800 + cells * (element == 2 ? 0.0154 : 0.0205) * (152.0 / sms);
 }
