@@ -347,6 +347,9 @@ static Several several_steps(const void *src, const void *dst, int nx, int ny, i
         }
     }
     if (dtype == LBGB_F64 || nx < 8 || ny < 16 || cells < 2048 || (m.ragged && es != 4)) return m;
+    // half precision: the march stands in for the pipelined kernel, which rounds the
+    // wall-density-1 lid's term on its own; the register kernel does not
+    if (dtype == LBGB_F16DEV && cells < g_tune.pipe_min_cells) return m;
     m.kind = Several::MARCH;
     m.most = cells >= 1500000 ? 4 : 2;
     return m;
