@@ -344,7 +344,10 @@ class BatchedLattice:
         self._buf[cur].copy_(saved)
         self._cur, self.steps_taken = cur, taken
         torch.cuda.synchronize(self.device)
-        return Replay(self, n)
+        replay = Replay(self, n)
+        # the graphs read these lists, which set_active lets go
+        replay.lists = (dict(self._tasks), dict(self._step_tasks))
+        return replay
 
     # ------------------------------------------------------------ diagnostics
     def shear_amplitudes(self, out=None):

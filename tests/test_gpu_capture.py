@@ -88,3 +88,21 @@ def test_batch_in_a_graph_of_the_callers(cuda, sizes, retired):
         torch.cuda.synchronize()
         for i in range(len(sizes)):
             assert torch.equal(a.populations(i), b.populations(i))
+
+
+@pytest.mark.parametrize("sizes", [SMALL, LARGE])
+def test_replay_keeps_its_lists(cuda, sizes):
+    """A graph of some of the instances stays good when others become active."""
+    a, b = make(sizes, "f32", "periodic", cuda), make(sizes, "f32", "periodic", cuda)
+    some = np.arange(len(sizes)) % 3 != 1
+    for x in (a, b):
+        x.set_active(some)
+    replay = a.capture(6)
+    a.set_active(np.ones(len(sizes), dtype=bool))
+    # what the allocator gives out next would lie where the lists were
+    rubbish = [torch.full((n,), -1, dtype=torch.int32, device=cuda) for n in (64, 256, 1024, 4096, 16384) for _ in range(50)]
+    replay()
+    b.step(6, SINGLE)
+    for i in range(len(sizes)):
+        assert torch.equal(a.populations(i), b.populations(i)), i
+    del rubbish
