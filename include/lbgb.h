@@ -275,11 +275,13 @@ LBGB_API int lbgb_batch_step(const void *src, void *dst, long long total_elems,
  * (*most, 1 to 8) and the tasks of a launch of `steps` steps (0: of *most) over
  * the n instances of sizes nx[b] x ny[b]: *n_tasks entries of four ints, of
  * which min(capacity, *n_tasks) are written to tasks (host memory).
- *   LBGB_BATCH_SINGLE  one step per launch only (lbgb_batch_step)
+ *   LBGB_BATCH_SINGLE  one step per launch only (lbgb_batch_step), also where
+ *                      that is expected to be faster (many narrow instances)
  *   LBGB_BATCH_MARCH   4 or 2 steps: large batches of 4-byte codes, every
  *                      instance at least 8 x 16
  *   LBGB_BATCH_TILE    1 to *most steps: small batches, every instance at least
  *                      2 x 2
+ * kind and *most do not depend on steps.
  * lbgb_batch_steps runs one launch over those tasks (device copy, 16-byte
  * aligned; a subset advances the instances whose tasks it holds).  Instances,
  * src, dst: as lbgb_batch_step.  No counterpart in the reference. */

@@ -190,7 +190,7 @@ inline double batch_march_cost(const MarchCount &c, int boundary, int dtype, int
 // 8000 of 16^2 174 and 43, 3000 of 32^2 116 and 60, 700 of 65^2 84 and 54, 2400 of
 // 64^2 176 and 170, 152 of 256^2 125 and 144; 68750 of 4^2 467 and 41, 4300 of 16^2
 // 28 and 22, 1100 of 32^2 14 and 22.  Over 455 batches of 1.3 to 10 M cells and
-// 507 of 10 k to 1.1 M the costs take the slower form in 6 %, by 9 % in the
+// 507 of 10 k to 1.1 M the costs take the slower form in 6 %, by 8 % in the
 // median; the factors lean to several steps, which also take fewer calls.
 inline double batch_tile_most(int dtype) { return dtype == LBGB_F64 ? 150000 : 1200000; }
 

@@ -396,8 +396,8 @@ class Lattice:
         ``step`` and with loading a state; read ``state`` after a replay."""
         if n <= 0 or n % 2:
             raise ValueError("capture: n must be a positive even number")
-        # load the kernel variant outside the capture: one step on a two-row
-        # copy with the same row length (same vector width, same template)
+        # load the library's code outside the capture: one step of two rows of this
+        # length (kernels of several steps load as they are recorded)
         warm = [torch.zeros((9, 2, self.ny), dtype=_RAW[self.storage], device=self.device) for _ in range(2)]
         _lib.call("lbgb_step_fused", warm[0].data_ptr(), warm[1].data_ptr(), 2, self.ny, self.bcode, self.omega,
                   self.u0, self.code, self._stream())
