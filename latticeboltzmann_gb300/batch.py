@@ -318,7 +318,7 @@ class BatchedLattice:
         lbgb_batch_plan; the same results bit for bit), or one per launch of
         ``config`` where one is given or several do not apply."""
         kind, several, singles = self._schedule(int(n)) if config is None else (None, [], int(n))
-        if several or kind == _lib.BATCH_MARCH:
+        if several or (singles > 0 and kind == _lib.BATCH_MARCH):
             lists = self._ready(kind, self._several()[1])
         for t in several:
             self._launch_steps(kind, t, lists[t])
